@@ -387,13 +387,13 @@ struct Walk {
     float P[3];  // cell-local position of the current cell's entry point
 };
 
-// walk_volume set-up (grid_traversal.pyx:42-118).  Returns false where the
+// walk_volume set-up (grid_traversal.pyx:42-118), general form.  Returns false where the
 // reference returns 0 before its loop.  Every float64 value it keeps is
 // computed from the same operands as the reference; float32 estimates only
 // decide comparisons whose outcome they prove (their margins exceed their
 // error bound by >= 80x), and the index and position of the entry point are
 // read from the bits of the float64 coordinate.
-YTGB_HD bool walk_setup(const BrickF &bf, const ytgb_brick *bp, const double *bounds, const Ray &r,
+YTGB_HD bool walk_setup_general(const BrickF &bf, const ytgb_brick *bp, const double *bounds, const Ray &r,
                         const float ifd[3], double max_t, long long kmax, Walk &w) {
     double le[3], re[3], idds[3];
     YTGB_UNROLL
@@ -510,6 +510,103 @@ YTGB_HD bool walk_setup(const BrickF &bf, const ytgb_brick *bp, const double *bo
     }
     w.enter_t = intersect_t;
     return true;
+}
+
+// The set-up for the common walk: float32 proves that the ray starts outside
+// the brick and enters it through the inside of one face (its hit point is
+// clearly on that face and clearly off the planes' other two).  The entry
+// axis is then a lane's own index, and the lanes of a warp form the two
+// float64 values of their entry face and the eight of their other two axes
+// together; the general set-up, unrolled over the axes, runs every axis' code
+// for the lanes that need it, up to 24 float64 instructions a walk for these
+// 16, and float64 (2 operations per SM and cycle) is what bounds the set-up.
+// With the warp's meeting after each walk (render kernel): 16 views of AMR
+// bricks in one batch 5.19 -> 4.50 ms, the 1024^2 AMR frame 1.57 -> 1.54 ms.
+// Returns 1 (walk), 0 (no cells) or -1 (float32 cannot tell: the general
+// set-up decides).
+YTGB_HD int walk_setup_face(const BrickF &bf, const ytgb_brick *bp, const double *bounds, const Ray &r,
+                            const float ifd[3], long long kmax, Walk &w) {
+    bool maybe_inside = true;
+    YTGB_UNROLL
+    for (int i = 0; i < 3; i++) {
+        const float m = 1e-5f * (fabsf(bf.lef[i]) + fabsf(bf.ref[i]) + fabsf(r.fpos[i]) + 1e-3f);
+        maybe_inside = maybe_inside && !(r.fpos[i] < bf.lef[i] - m) && !(r.fpos[i] > bf.ref[i] + m);
+    }
+    int direction = -1;
+    bool sure = !maybe_inside;
+    YTGB_UNROLL
+    for (int i = 0; i < 3; i++) {
+        if (r.step[i] == 0) continue;
+        const int x = (i + 1) % 3, y = (i + 2) % 3;
+        // (the general set-up's estimates and margins)
+        const float e = r.step[i] > 0 ? bf.lef[i] : bf.ref[i];
+        const float a0 = fabsf(e) + fabsf(r.fpos[i]);
+        const float tlf = (e - r.fpos[i]) * ifd[i];
+        const float qx = r.fpos[x] + tlf * r.fdir[x];
+        const float qy = r.fpos[y] + tlf * r.fdir[y];
+        const float sx = 1e-5f * (a0 * fabsf(r.fdir[x] * ifd[i]) + fabsf(tlf * r.fdir[x]) + fabsf(r.fpos[x]) +
+                                  fabsf(bf.lef[x]) + fabsf(bf.ref[x]) + 1e-3f);
+        const float sy = 1e-5f * (a0 * fabsf(r.fdir[y] * ifd[i]) + fabsf(tlf * r.fdir[y]) + fabsf(r.fpos[y]) +
+                                  fabsf(bf.lef[y]) + fabsf(bf.ref[y]) + 1e-3f);
+        const float st = 1e-5f * (a0 * fabsf(ifd[i]) + fabsf(tlf) + 1e-3f);
+        const bool off = qx < bf.lef[x] - sx || qx > bf.ref[x] + sx || qy < bf.lef[y] - sy || qy > bf.ref[y] + sy ||
+                         tlf < -st;
+        const bool on = qx > bf.lef[x] + sx && qx < bf.ref[x] - sx && qy > bf.lef[y] + sy && qy < bf.ref[y] - sy;
+        sure = sure && (off || (on && direction < 0));
+        direction = off ? direction : i;
+    }
+    if (!sure) return -1;
+    if (direction < 0) return 0;  // off every face it could enter
+    const int i = direction, x = i == 2 ? 0 : i + 1, y = i == 0 ? 2 : i - 1;
+    const int si = r.step[i];
+    const double tl = dmul(dsub(si > 0 ? ldg(&bp->left_edge[i]) : ldg(&bp->right_edge[i]), r.pos[i]), r.iv[i]);
+    const long long kint = dkey(tl);
+    if (!(kint >= 0 && kint < kmax)) return 0;  // !(0 <= intersect_t < max_t) (max_t <= 1)
+    w.enter_t = tl;
+    // the entry cell and position on the other two axes
+    int cx, cy;
+    float px, py;
+    YTGB_UNROLL
+    for (int k = 0; k < 2; k++) {
+        const int q = k ? y : x;
+        const double le = ldg(&bp->left_edge[q]);
+        const double tx = dadd(dmul(tl, r.dir[q]), r.pos[q]);
+        const double ty = dmul(dsub(tx, le), ldg(&bp->idds[q]));
+        const long long tb = dbits(ty);
+        if (!(tb > 0 && tb < 0x41d0000000000000LL)) return -1;
+        if (k) split_floor(tb, cy, py);
+        else split_floor(tb, cx, px);
+    }
+    const int dn = i == 0 ? bf.dims[0] : (i == 1 ? bf.dims[1] : bf.dims[2]);
+    const int ci = si > 0 ? 0 : dn - 1;
+    const float pi = si > 0 ? 0.0f : 1.0f;
+    w.cur[0] = i == 0 ? ci : (i == 1 ? cy : cx);
+    w.cur[1] = i == 1 ? ci : (i == 2 ? cy : cx);
+    w.cur[2] = i == 2 ? ci : (i == 0 ? cy : cx);
+    w.P[0] = i == 0 ? pi : (i == 1 ? py : px);
+    w.P[1] = i == 1 ? pi : (i == 2 ? py : px);
+    w.P[2] = i == 2 ? pi : (i == 0 ? py : px);
+    const long long boff = ldg(&bp->bounds_offset);
+    int aoff = 0;
+    bool in = true;
+    YTGB_UNROLL
+    for (int q = 0; q < 3; q++) {
+        const int dims = bf.dims[q];
+        const int k = r.step[q] > 0 ? w.cur[q] + 1 : w.cur[q];
+        in = in && (unsigned)w.cur[q] < (unsigned)dims;
+        if (in) w.tmax[q] = r.step[q] != 0 ? dmul(dsub(ldg(bounds + boff + aoff + k), r.pos[q]), r.iv[q]) : 1e60;
+        aoff += dims + 1;
+    }
+    return in ? 1 : -1;
+}
+
+// walk_volume set-up: the common walk's form where float32 proves it, else
+// the general one.
+YTGB_HD bool walk_setup(const BrickF &bf, const ytgb_brick *bp, const double *bounds, const Ray &r,
+                        const float ifd[3], double max_t, long long kmax, Walk &w) {
+    const int s = walk_setup_face(bf, bp, bounds, r, ifd, kmax, w);
+    if (__builtin_expect(s < 0, 0)) return walk_setup_general(bf, bp, bounds, r, ifd, max_t, kmax, w);
+    return s > 0;
 }
 
 // ---- compensated float32 accumulation -------------------------------------

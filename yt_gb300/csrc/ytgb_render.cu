@@ -168,13 +168,15 @@ __device__ __forceinline__ void warp_tile(const ytgb_render_args &a, int bx, int
         nsel += __popc(bal);
         if (nsel > SEL_CAP - 32 || base + 32 >= n_order) {
             __syncwarp();
-            for (int j = 0; active && j < nsel; j++) {
+            for (int j = 0; j < nsel; j++) {
                 const int kk = sel[j];
                 const int4 rc = __ldg(rects + kk);
-                if (vi < rc.x || vi >= rc.y || vj < rc.z || vj >= rc.w) continue;
-                walk_brick<MODE, VAR, TG>(a, tab, r, __ldg(a.order + kk), st);
+                if (active && vi >= rc.x && vi < rc.y && vj >= rc.z && vj < rc.w)
+                    walk_brick<MODE, VAR, TG>(a, tab, r, __ldg(a.order + kk), st);
+                // every lane takes the next brick's set-up together
+                __syncwarp();
             }
-            __syncwarp();  // the list is rewritten by the next passes
+            // (the list is rewritten by the next passes)
             nsel = 0;
         }
     }
