@@ -97,3 +97,46 @@ extern "C" void check_setup(long long n, int aim, unsigned long long seed, long 
         if (!same) out[2]++;
     }
 }
+
+// Runs of integer steps (run_axis) against float64 adds: from each start a
+// walk of steps on one axis, taken as the cell loop takes them -- adds of the
+// run's increment below its limit, the float64 add and a new run at it.
+// ties: tdelta with few significant bits (exact halves); left: the brick's
+// remaining steps.  Returns the mismatches; looks: the steps taken in full.
+extern "C" long long check_runs(long long n, int steps, int ties, unsigned long long seed, long long *looks) {
+    std::mt19937_64 g(seed);
+    std::uniform_real_distribution<double> u(0.0, 1.0);
+    const long long kmax = dkey(1.0);
+    long long bad = 0;
+    *looks = 0;
+    for (long long k = 0; k < n; k++) {
+        double x = std::pow(2.0, -14.0 * u(g)) * 0.999, d = std::pow(2.0, -2.0 - 14.0 * u(g));
+        if (ties) {
+            long long b = dbits(d);
+            b &= ~((1LL << (40 + g() % 12)) - 1);
+            d = dfrom(b);
+            b = dbits(x) & ~((1LL << (g() % 52)) - 1);
+            x = dfrom(b | (long long)(g() % 2));
+        }
+        const float v = (float)(1.0 / d);
+        int left = 1 + (int)(g() % (2 * steps));
+        long long t = dbits(x), at = kmax, inc = 0;
+        double ref = x;
+        if (t < kmax) inc = run_axis(t, dbits(d), v, left, at);
+        for (int j = 0; j < steps && left > 0 && t < kmax; j++, left--) {
+            if (t < at) {
+                if (left == 1) { bad++; break; }  // the leaving step must be looked at
+                t += inc;
+            } else {
+                ++*looks;
+                t = dbits(dfrom(t) + d);
+                at = kmax;
+                inc = 0;
+                if (left > 1 && t < kmax) inc = run_axis(t, dbits(d), v, left - 1, at);
+            }
+            ref = ref + d;
+            if (t != dbits(ref)) { bad++; break; }
+        }
+    }
+    return bad;
+}

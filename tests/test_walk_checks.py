@@ -5,7 +5,6 @@ import os
 import subprocess
 from pathlib import Path
 
-import numpy as np
 import pytest
 
 ROOT = Path(__file__).resolve().parent.parent
@@ -33,3 +32,17 @@ def test_setup_by_entry_face_equals_general(checks, aim, least):
     decided, left, wrong = out
     assert wrong == 0
     assert decided + left == n and decided >= least * n
+
+
+@pytest.mark.parametrize("steps", [1, 7, 64, 2000])
+@pytest.mark.parametrize("ties", [0, 1])
+def test_runs_of_steps_equal_float64_adds(checks, steps, ties):
+    """tmax after every step of a run is the float64 sum's bits, across
+    binades and exact halves, and the step that leaves the brick is never
+    inside a run."""
+    n = 2_000_000 // (steps + 10)
+    looks = C.c_longlong()
+    checks.check_runs.restype = C.c_longlong
+    bad = checks.check_runs(C.c_longlong(n), steps, ties, C.c_ulonglong(5 + steps), C.byref(looks))
+    assert bad == 0
+    assert looks.value > 0

@@ -18,7 +18,8 @@
 //   * per cell `tmax += tdelta` runs as an integer add on the bit pattern
 //     (float64 only when tmax leaves its binade) and `exit_t - enter_t` as
 //     an integer difference converted to float32 once, by 32-bit integer
-//     conversions (a 64-bit conversion runs on the float64 pipe);
+//     conversions (a 64-bit conversion runs on the float64 pipe), with one
+//     limit on tmax in place of a step's other tests;
 //   * the sample position is tracked in float32, in cell-local coordinates
 //     reset exactly on the axis the walk steps along;
 //   * bricks a ray clearly misses, faces it clearly does not enter through,
@@ -67,22 +68,33 @@ template <> struct TileShape<1> { static constexpr int X = 16, Y = 8; };
 template <> struct TileShape<2> { static constexpr int X = 4, Y = 32; };
 constexpr int BLOCK = 128;
 constexpr int NWARP = BLOCK / 32;
-// Resident blocks per SM the kernels are compiled for.  The per-ray walk is
-// latency-bound (dependent integer and float64 steps), so warps per SM
-// count for more than registers.  The single-view kernel takes 6 (80
-// registers, a few spills in the per-walk state): on the 1024^2 AMR frame
-// 1.199 ms against 1.234 ms at 5 (96 registers, no spills), and the
-// projections 3-6 % faster.  The persistent batch kernel, whose loop keeps
-// more state, takes 5: the 64-view batch runs 32.7 ms against 33.2 ms at
-// 6.  The single-view kernel's float64-range-decision variants (V_REF, the
-// served form's) keep 5 too: at 80 registers their rare float64 path
-// spilled ~1 KB a thread and the served frame ran 2.46 ms against 2.03 ms
-// at 96.  Images are identical at every setting.  YTGB_MIN_BLOCKS sets both
-// (a second build at another budget, for the bit-identity test).
+// Resident blocks per SM the kernels are compiled for: warps hide the walk's
+// latencies, registers spare it spills.  Measured for each sampler (kernel
+// time, the other choices beside it):
+//   cell samplers (projection, maximum), whose loop holds little: 7 blocks,
+//     72 registers: 6.38 ms and 651 us (6: 6.55 and 690; 8: 6.68 and 652; 5:
+//     7.01 and 756) for 512^3 at 2048^2 and 255^3 at 1023x779;
+//   interpolated projection: 6, 80 registers: 1.026 ms (5: 1.023, 7: 1.057);
+//   ColorTransferFunction rendering: 5, 96 registers: 1.362 ms on the 1024^2
+//     AMR frame (6: 1.406);
+//   with float64 range decisions (V_REF), whose rare path needs the most: 4,
+//     128 registers: 505 us on a 701x1003 AMR frame (5: 545);
+//   other table sets, the light source and the traversal trace: 6.
+// The persistent batch kernel, whose loop keeps more state: 5 (4.56 ms for 16
+// views; 4: 4.66, 6: 4.80).  Images are identical at every setting.
+// YTGB_MIN_BLOCKS sets all (a second build at another budget, for the
+// bit-identity test).
 #ifdef YTGB_MIN_BLOCKS
-constexpr int MIN_BLOCKS = YTGB_MIN_BLOCKS, BATCH_MIN_BLOCKS = YTGB_MIN_BLOCKS;
+constexpr int min_blocks(int, int) { return YTGB_MIN_BLOCKS; }
+constexpr int BATCH_MIN_BLOCKS = YTGB_MIN_BLOCKS;
 #else
-constexpr int MIN_BLOCKS = 6, BATCH_MIN_BLOCKS = 5;
+constexpr int min_blocks(int mode, int var) {
+    return (var & V_REF) ? 4
+           : mode == MODE_PROJ || mode == MODE_MIP ? 7
+           : mode == MODE_VR && (var & V_CTF) ? 5
+                                              : 6;
+}
+constexpr int BATCH_MIN_BLOCKS = 5;
 #endif
 
 // Selected bricks a warp holds before walking them (flushed in order when
@@ -173,7 +185,9 @@ __device__ __forceinline__ void warp_tile(const ytgb_render_args &a, int bx, int
                 const int4 rc = __ldg(rects + kk);
                 if (active && vi >= rc.x && vi < rc.y && vj >= rc.z && vj < rc.w)
                     walk_brick<MODE, VAR, TG>(a, tab, r, __ldg(a.order + kk), st);
-                // every lane takes the next brick's set-up together
+                // every lane takes the next brick's set-up together (left to
+                // itself the compiler let lanes that had finished a walk go
+                // on alone: half the lanes idle)
                 __syncwarp();
             }
             // (the list is rewritten by the next passes)
@@ -188,7 +202,7 @@ __device__ __forceinline__ void warp_tile(const ytgb_render_args &a, int bx, int
         } else {
 #pragma unroll
             for (int c = 0; c < 4; c++)
-                if (st.touched & (1u << c)) img[c] = (double)st.xh[c] + (double)st.xl[c];
+                if (st.touched & (1u << c)) img[c] = image_value(st, c);
         }
     }
     if (a.counters) {
@@ -208,8 +222,8 @@ __device__ __forceinline__ void warp_tile(const ytgb_render_args &a, int bx, int
 
 // One view, one tile per block (four warps of 32 pixels).
 template <int MODE, int VAR, int TS>
-__global__ void __launch_bounds__(BLOCK, (VAR & V_REF) ? BATCH_MIN_BLOCKS : MIN_BLOCKS) render_kernel(const ytgb_render_args a, unsigned long long *hashes,
-                                                       long long *counts) {
+__global__ void __launch_bounds__(BLOCK, min_blocks(MODE, VAR))
+render_kernel(const ytgb_render_args a, unsigned long long *hashes, long long *counts) {
     extern __shared__ float4 s_tab[];
     __shared__ TileSmem sm;
     if (MODE == MODE_VR || MODE == MODE_LIGHT) {
