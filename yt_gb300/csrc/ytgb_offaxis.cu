@@ -25,6 +25,7 @@
 // float64 fused multiply-adds, a few roundings per contribution.  Cells whose rows exceed the table take the
 // reference's per-subcell loop (with atomics) instead.
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdint>
 #include <string>
 
@@ -355,9 +356,399 @@ __global__ void __launch_bounds__(OA_BLOCK) offaxis_kernel(const ytgb_offaxis_ar
     }
 }
 
+
+// ---- splatting by summed stamps --------------------------------------------
+//
+// A subcell's mass goes to its left pixel with dv and to its right pixel with
+// 1 - dv, so the mass of a cell in the pixels (<= P, <= Q) is the stamp's sum
+// over the subcells whose right pixels are within, plus the dv of the one
+// column and the one row that P and Q cut: a bilinear look-up in the stamp's
+// summed-area table.  A pixel's mass is the difference of four such corners.
+// The subcell kernel above spends some 30 to 90 float64 operations on a pixel,
+// at 2 per SM and cycle its bound (float64 pipe 90 % busy); a corner takes
+// three products of 64-bit integers, on the integer pipe.
+//
+// The table is in fixed point, modulo 2^64, in units of 2^-(62 + s) of the
+// stamp's unit sum (level_shift): only differences are used, and those that
+// occur (one subcell column's or row's sum, a pixel's mass) fit 64 bits, so
+// that they are exact; in float64 the corners' cancellation would cost a large
+// cell's pixels three digits.  Entries are rounded to half a unit and the
+// products down, so that a pixel is within four units: 2e-17 of a pixel's
+// share of the cell, at every level.
+//
+// The subcell boundaries, their pixels and dv are formed by the reference's
+// float64 operations, once per pixel boundary and axis.  A warp takes a few cells,
+// strided over the list so that each batch has cells of all sizes: first one
+// lane per cell for what depends on the cell alone, then one lane per pixel
+// boundary of as many cells as the table in shared memory holds, then the
+// pixels cell by cell, lanes over the columns and groups of lanes over the rows.
+// Measured (197,000 cells of levels 5-9 at 1024^2, 38 pixels to 2): 5.17 ms by
+// the subcell kernel, 1.02 with 32 cells a batch and float64 products and
+// conversions, 0.93 with the conversions on the integer pipe, 0.83 with one
+// block per four batches (the scheduler evens out the last wave), 0.74 with 6
+// blocks per SM and 16 cells, 0.73 with the products on the integer pipe, 0.69
+// with 8 cells and 7 blocks (12 and 6: 0.70; 6 and 6: 0.71).  Now the float64
+// pipe (boundaries and their divisions) and the integer pipe are each about
+// 40 % busy and issue 55 %; with plain stores for the atomics it is no faster.
+constexpr int OS_CAP = 520;   // pixel boundaries held per warp: a cell of 258 pixels each way
+constexpr int OS_CELLS = 8;   // cells of a warp's batch
+constexpr int OS_WARPS = 4;
+constexpr int OS_BLOCKS = 7;  // resident blocks per SM: 72 registers
+
+// s of a level of jm x km subcells.  A row or column of subcells holds at
+// most sqrt(6) / min(jm, km) of the sum (the largest plane section of a cube
+// is sqrt(2) of a face, across a cube 1 / sqrt(3) of the stamp's width) and a
+// subcell 3 sqrt(3) / (jm km) (the cube's diagonal); the level is chosen with
+// fewer than 8 subcells per pixel along the longer image axis
+// (image_utilities.pyx:92-99).  So the former stay below 2^64 units and a
+// pixel, which may hold the whole sum, at most 2^62 (with a margin of 1.3 for
+// the stamp's own discretisation).
+__device__ __forceinline__ int level_shift(int jm, int km, int nx, int ny) {
+    const int lg = 31 - __clz(min(jm, km));
+    const float n = (float)max(nx, ny), px = 8.0f * n / (float)nx, py = 8.0f * n / (float)ny;
+    const float mass = 1.3f * 5.2f * px * py / ((float)jm * (float)km);
+    int s = 0;
+    while (s < lg && mass * (float)(1ll << (s + 1)) <= 1.0f) s++;
+    return s;
+}
+
+struct SplatCell {
+    double x, y, dlx, dly, cq, cw;
+    float bx, by, sx, sy;  // estimate of the subcell at a pixel boundary: ceil(s * P + b) - 1
+    int depth, jm, km, unit;  // unit: 2^-unit is the table's
+    int P0, Pn, Q0, Qn;    // first pixel and number of pixels, per axis (0: nothing to do)
+};
+
+struct SplatSmem {
+    SplatCell cell[OS_CELLS];
+    unsigned long long w[OS_CAP];  // dv of the cut subcell, 2^-64
+    int at[OS_CAP];                // its index
+    int off[OS_CELLS], who[OS_CELLS];          // the packed cells' first entries, and which cells they are
+};
+
+// floor(a b / 2^64)
+__device__ __forceinline__ unsigned long long scale64(unsigned long long a, unsigned long long b) {
+    return __umul64hi(a, b);
+}
+
+// x in [0, 1] in units of 2^-64 (1 as the largest value), anything else clipped
+__device__ __forceinline__ unsigned long long unit64(double x) {
+    const long long b = dbits(x);
+    if (b <= 0 || b > 0x7ff0000000000000LL) return 0ull;  // negative, zero, NaN
+    if (b >= 0x3ff0000000000000LL) return ~0ull;
+    const int sh = (int)(b >> 52) - 1011;  // x = m 2^(e - 1075)
+    const unsigned long long m = (unsigned long long)((b & MANT52) | (1LL << 52));
+    return sh >= 0 ? m << sh : (sh > -53 ? m >> -sh : 0ull);
+}
+
+// (double)v for 0 <= v < 2^31 and the truncation of |x| < 2^31 (others by the
+// conversion), on the integer pipe: the conversions take the float64 pipe
+__device__ __forceinline__ double to_double(int v) {
+    const int lead = 31 - __clz(v);
+    const unsigned m = (unsigned)v << (31 - lead);  // 1 at bit 31
+    return v == 0 ? 0.0 : __hiloint2double((int)(((unsigned)(lead + 1023) << 20) | ((m >> 11) & 0xfffffu)), (int)(m << 21));
+}
+__device__ __forceinline__ int truncate(double x) {
+    const int e = ((__double2hiint(x) >> 20) & 0x7ff) - 1023;
+    if (e < 0) return 0;
+    if (e > 30) return __double2int_rz(x);
+    const unsigned long long m = ((unsigned long long)dbits(x) & MANT52) | (1ull << 52);
+    const int v = (int)(m >> (52 - e));
+    return __double2hiint(x) < 0 ? -v : v;
+}
+
+// Subcell boundary i as `boundary` forms it: i - m / 2 is exact, so its
+// product with d is that of 2 i - m with d / 2 (dh, exact)
+__device__ __forceinline__ double boundary_half(int i, int m, double dh, double x, double N) {
+    const int k = 2 * i - m;
+    const double a = to_double(k < 0 ? -k : k);
+    return ytgb::dmul(ytgb::dadd(ytgb::dmul(k < 0 ? -a : a, dh), x), N);
+}
+
+// The subcell that pixel boundary P (the right edge of pixel P; -1: of what
+// lies left of pixel 0) cuts: the first whose right boundary truncates past
+// P, with its dv where its left boundary does not (image_utilities.pyx:
+// 110-120 and 124-138); m and 0 past the last.
+__device__ __forceinline__ void cut_subcell(int P, int m, double d, double x, int n, float s, float b, int &at,
+                                            unsigned long long &w) {
+    const double dh = ytgb::dmul(d, 0.5), N = to_double(n);
+    const float est = ceilf(ffma(s, (float)(P < 0 ? -1 : P + 1), b));
+    int j = (int)fminf(fmaxf(est - 1.0f, 0.0f), (float)(m - 1));
+    double b0 = boundary_half(j, m, dh, x, N), b1 = boundary_half(j + 1, m, dh, x, N);
+    int e0 = truncate(b0), e1 = truncate(b1);
+    // (the estimate is within a subcell or two: float32 of P * subcells per pixel)
+    while (j > 0 && e0 > P) {
+        j--;
+        b1 = b0;
+        e1 = e0;
+        b0 = boundary_half(j, m, dh, x, N);
+        e0 = truncate(b0);
+    }
+    while (j < m && !(e1 > P)) {
+        j++;
+        b0 = b1;
+        e0 = e1;
+        b1 = boundary_half(j + 1, m, dh, x, N);
+        e1 = truncate(b1);
+    }
+    at = j;
+    w = j < m && e0 <= P ? unit64(ytgb::ddiv(ytgb::dsub(to_double(e1), b0), ytgb::dsub(b1, b0))) : 0ull;
+}
+
+// A float64 factor as a 64-bit mantissa (1 at bit 63), exponent and sign, for
+// scaled_mass; ok false (subnormal, zero, infinite, NaN) where the product is
+// left to float64.
+struct Factor {
+    unsigned long long m;
+    long long eb;  // sign and biased exponent field, shifted into place
+    bool ok;
+};
+__device__ __forceinline__ Factor factor_of(double x) {
+    const long long b = dbits(x);
+    const int e = (int)(b >> 52) & 0x7ff;
+    Factor f;
+    f.m = ((unsigned long long)(b & MANT52) | (1ull << 52)) << 11;
+    f.eb = b & ~MANT52;
+    f.ok = e > 200 && e < 1800;  // (the product's exponent stays inside the field)
+    return f;
+}
+
+// x times mass 2^-unit, where m is mass shifted to have 1 at bit 63 and `down`
+// = unit - 63 + the shift: the 128-bit product's upper half, rounded to 53 bits
+// (ties away from zero; the part dropped before is below 2^-63 of the value),
+// on the integer pipe where a float64 product takes the float64 pipe 64 cycles.
+__device__ __forceinline__ double scaled_mass(unsigned long long m, int down, const Factor &f) {
+    unsigned long long p = __umul64hi(m, f.m);  // in [2^62, 2^64)
+    const int up = (int)(p >> 63);
+    p = up ? p : p << 1;
+    const unsigned long long r = ((p & 0x7fffffffffffffffull) + 0x400ull) >> 11;  // a carry adds to the exponent
+    return dfrom(f.eb + (long long)r + ((long long)(up - down) << 52));
+}
+
+// the table's value at a corner: rows at, at + 1 and columns b0, b1 (two
+// neighbours, or twice the last)
+__device__ __forceinline__ unsigned long long corner(const unsigned long long *__restrict__ S, int stride, int m,
+                                                     int at, unsigned long long wa, int b0, int b1,
+                                                     unsigned long long wb) {
+    const unsigned long long *r0 = S + (long long)at * stride, *r1 = S + (long long)min(at + 1, m) * stride;
+    const unsigned long long u0 = __ldg(r0 + b0), u1 = __ldg(r0 + b1), v0 = __ldg(r1 + b0), v1 = __ldg(r1 + b1);
+    const unsigned long long u = u0 + scale64(u1 - u0, wb), v = v0 + scale64(v1 - v0, wb);
+    return u + scale64(v - u, wa);
+}
+
+__global__ void __launch_bounds__(OS_WARPS * 32, OS_BLOCKS)
+splat_kernel(const ytgb_offaxis_args a, const unsigned long long *__restrict__ sums, int32_t *error) {
+    __shared__ SplatSmem s_all[OS_WARPS];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    SplatSmem &sm = s_all[wib];
+    const int nx = a.nx, ny = a.ny;
+    const long long npix = (long long)nx * ny;
+    const double sq3 = ytgb::dsqrt(3.0);
+    const double sq3x4 = ytgb::dmul(4.0, sq3);
+    const double nmax = nx > ny ? (double)nx : (double)ny;  // fmax(Nx, Ny)
+    const long long batches = (a.n + OS_CELLS - 1) / OS_CELLS;
+    const int stride = a.nsy + 1;
+    for (long long bt = (long long)blockIdx.x * OS_WARPS + wib; bt < batches; bt += (long long)gridDim.x * OS_WARPS) {
+        // ---- one lane per cell
+        const long long c = bt + (long long)lane * batches;
+        int Pn = 0, Qn = 0;
+        bool wide = false;
+        if (lane < OS_CELLS && c < a.n) {
+            const double dx = __ldg(a.dxp + c), w = __ldg(a.weight + c), q = __ldg(a.qty + c);
+            const double X0 = __ldg(a.xp + 3 * c), X1 = __ldg(a.xp + 3 * c + 1), X2 = __ldg(a.xp + 3 * c + 2);
+            if (!(dx > 0.0) || !isfinite(dx)) {
+                if (error) atomicCAS(error, 0, YTGB_DEVERR_BAD_CELL);
+            } else {
+                SplatCell &sc = sm.cell[lane];
+                const double cmw = ytgb::dmul(dx, sq3);
+                const double x = ytgb::dadd(ytgb::dadd(ytgb::dadd(ytgb::dmul(a.rot[0], X0), ytgb::dmul(a.rot[1], X1)), ytgb::dmul(a.rot[2], X2)), 0.5);
+                const double y = ytgb::dadd(ytgb::dadd(ytgb::dadd(ytgb::dmul(a.rot[3], X0), ytgb::dmul(a.rot[4], X1)), ytgb::dmul(a.rot[5], X2)), 0.5);
+                const double half = ytgb::dmul(cmw, 0.5);  // cmw / 2, exactly
+                const double dx3 = ytgb::dmul(ytgb::dmul(ytgb::dmul(ytgb::dmul(dx, dx), dx), (double)nx), (double)ny);
+                const double lx = ytgb::dsub(x, half), rx = ytgb::dadd(x, half), ly = ytgb::dsub(y, half), ry = ytgb::dadd(y, half);
+                const int jmin = max(__double2int_rz(floor(ytgb::dmul(lx, (double)nx))), 0);
+                const int jmax = max(__double2int_rz(ceil(ytgb::dmul(rx, (double)nx))), nx - 1);
+                const int kmin = min(__double2int_rz(floor(ytgb::dmul(ly, (double)ny))), 0);
+                const int kmax = max(__double2int_rz(ceil(ytgb::dmul(ry, (double)ny))), ny - 1);
+                if (jmax == jmin + 1 && kmax == kmin + 1) {  // image_utilities.pyx:83-87, the cell inside one pixel
+                    const long long idx = (long long)jmin * nx + kmin;
+                    if (idx >= 0 && idx < npix) {
+                        atomicAdd(a.buffer + idx, ytgb::dmul(q, dx3));
+                        atomicAdd(a.buffer_weight + idx, ytgb::dmul(w, dx3));
+                    }
+                } else {
+                    // :92-99: the stamp level with at least 4 subcells per pixel diagonal
+                    const double v = ytgb::dmul(ytgb::dmul(sq3x4, dx), nmax);
+                    int depth = v > 1.0 ? ceil_log2_above1(v) : 1;
+                    depth = depth < 1 ? 1 : (depth > a.max_depth - 1 ? a.max_depth - 1 : depth);
+                    const int jm = min(a.nsx, 1 << depth), km = min(a.nsy, 1 << depth);
+                    // cmw / 2^depth is an exact scaling
+                    const double pw = dfrom((long long)(1023 - depth) << 52);
+                    sc.dlx = jm == (1 << depth) ? ytgb::dmul(cmw, pw) : ytgb::ddiv(cmw, (double)jm);
+                    sc.dly = km == (1 << depth) ? ytgb::dmul(cmw, pw) : ytgb::ddiv(cmw, (double)km);
+                    sc.x = x;
+                    sc.y = y;
+                    sc.cq = ytgb::dmul(dx3, q);
+                    sc.cw = ytgb::dmul(dx3, w);
+                    sc.depth = depth;
+                    sc.jm = jm;
+                    sc.km = km;
+                    sc.unit = 62 + level_shift(jm, km, nx, ny);
+                    // pixels the cell can reach (the boundaries are nondecreasing)
+                    const int P0 = max(__double2int_rz(boundary(0, jm, sc.dlx, x, nx)), 0);
+                    const int P1 = min(__double2int_rz(boundary(jm, jm, sc.dlx, x, nx)), nx - 1);
+                    const int Q0 = max(__double2int_rz(boundary(0, km, sc.dly, y, ny)), 0);
+                    const int Q1 = min(__double2int_rz(boundary(km, km, sc.dly, y, ny)), ny - 1);
+                    sc.P0 = P0;
+                    sc.Q0 = Q0;
+                    const float fdx = (float)sc.dlx, fdy = (float)sc.dly;
+                    sc.sx = 1.0f / ((float)nx * fdx);
+                    sc.sy = 1.0f / ((float)ny * fdy);
+                    sc.bx = 0.5f * (float)jm - (float)x / fdx;
+                    sc.by = 0.5f * (float)km - (float)y / fdy;
+                    if (P0 <= P1 && Q0 <= Q1 && isfinite(x) && isfinite(y)) {
+                        Pn = P1 - P0 + 1;
+                        Qn = Q1 - Q0 + 1;
+                        wide = (long long)Pn + Qn + 2 > OS_CAP;
+                    }
+                    sc.Pn = Pn;
+                    sc.Qn = Qn;
+                }
+            }
+        }
+        __syncwarp();
+        // ---- cells wider than the table holds: the reference's own loop
+        for (unsigned m = __ballot_sync(0xffffffffu, wide); m; m &= m - 1) {
+            const SplatCell &sc = sm.cell[__ffs(m) - 1];
+            const long long cc = bt + (long long)(__ffs(m) - 1) * batches;
+            const double dx = __ldg(a.dxp + cc);
+            cell_direct(a, lane, sc.depth, sc.jm, sc.km, sc.dlx, sc.dly, sc.x, sc.y,
+                        ytgb::dmul(ytgb::dmul(ytgb::dmul(ytgb::dmul(dx, dx), dx), (double)nx), (double)ny),
+                        __ldg(a.weight + cc), __ldg(a.qty + cc));
+        }
+        const int need = Pn > 0 && !wide ? Pn + Qn + 2 : 0;  // this lane's cell's pixel boundaries
+        unsigned left = __ballot_sync(0xffffffffu, need > 0);
+        while (left) {
+            // ---- the first cells whose boundaries fit the table
+            int incl = (left >> lane) & 1u ? need : 0;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += v;
+            }
+            const bool in = ((left >> lane) & 1u) && incl <= OS_CAP;
+            const unsigned take = __ballot_sync(0xffffffffu, in);
+            const int total = __reduce_max_sync(0xffffffffu, in ? incl : 0);
+            const int rank = __popc(take & ((1u << lane) - 1u)), n_take = __popc(take);
+            if (in) {
+                sm.off[rank] = incl - need;
+                sm.who[rank] = lane;
+            }
+            __syncwarp();
+            // ---- one lane per pixel boundary
+            for (int t = lane; t < total; t += 32) {
+                int lo = 0, hi = n_take - 1;
+                while (lo < hi) {
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (sm.off[mid] <= t) lo = mid;
+                    else hi = mid - 1;
+                }
+                const SplatCell &sc = sm.cell[sm.who[lo]];
+                const int k = t - sm.off[lo];
+                const bool col = k > sc.Pn;  // rows' boundaries first, then the columns'
+                const int P = col ? sc.Q0 - 1 + (k - sc.Pn - 1) : sc.P0 - 1 + k;
+                int at;
+                unsigned long long w;
+                cut_subcell(P, col ? sc.km : sc.jm, col ? sc.dly : sc.dlx, col ? sc.y : sc.x, col ? ny : nx,
+                            col ? sc.sy : sc.sx, col ? sc.by : sc.bx, at, w);
+                sm.at[t] = at;
+                sm.w[t] = w;
+            }
+            __syncwarp();
+            // ---- the pixels, cell by cell
+            for (int i = 0; i < n_take; i++) {
+                const SplatCell &sc = sm.cell[sm.who[i]];
+                const int o = sm.off[i], rows = sc.Pn, jm = sc.jm, km = sc.km;
+                const unsigned long long *S = sums + (long long)sc.depth * (a.nsx + 1) * stride;
+                const Factor fq = factor_of(sc.cq), fw = factor_of(sc.cw);
+                const bool plain = fq.ok && fw.ok;
+                const int *ra = sm.at + o, *ca = ra + rows + 1;
+                const unsigned long long *rw = sm.w + o, *cw = rw + rows + 1;
+                for (int q0 = 0; q0 < sc.Qn; q0 += 31) {
+                    // lanes over the column boundaries q0 .. q0 + nb - 1, groups of
+                    // them over the rows
+                    const int nb = min(32, sc.Qn + 1 - q0);
+                    const int groups = 32 / nb, g = lane / nb, q = q0 + lane - g * nb;
+                    const bool on = g < groups;
+                    const int b = on ? ca[q] : 0;
+                    const int b1 = min(b + 1, km);
+                    const unsigned long long wb = on ? cw[q] : 0ull;
+                    const int r0 = on ? g * rows / groups : 0, r1 = on ? (g + 1) * rows / groups : 0;
+                    const int steps = (rows + groups - 1) / groups;
+                    const int Q = sc.Q0 + q - 1;  // the pixel left of this boundary
+                    const bool px = on && lane > g * nb;
+                    unsigned long long prev = on ? corner(S, stride, jm, ra[r0], rw[r0], b, b1, wb) : 0ull;
+                    for (int k = 0; k < steps; k++) {
+                        const int r = min(r0 + k + 1, r1);
+                        const unsigned long long G = on ? corner(S, stride, jm, ra[r], rw[r], b, b1, wb) : 0ull;
+                        const unsigned long long d = G - prev;
+                        prev = G;
+                        const unsigned long long dl = __shfl_up_sync(0xffffffffu, d, 1);
+                        const long long mass = (long long)(d - dl);  // (rounding may leave a few units below 0)
+                        if (px && r0 + k < r1 && mass > 0) {
+                            const long long idx = (long long)(sc.P0 + r0 + k) * nx + Q;
+                            if (idx < npix) {
+                                const int sh = __clzll(mass);
+                                const unsigned long long m = (unsigned long long)mass << sh;
+                                const int down = sc.unit - 63 + sh;
+                                double vq, vw;
+                                if (plain) {
+                                    vq = scaled_mass(m, down, fq);
+                                    vw = scaled_mass(m, down, fw);
+                                } else {
+                                    const double f = dfrom(dbits((double)mass) - ((long long)sc.unit << 52));
+                                    vq = ytgb::dmul(f, sc.cq);
+                                    vw = ytgb::dmul(f, sc.cw);
+                                }
+                                atomicAdd(a.buffer + idx, vq);
+                                atomicAdd(a.buffer_weight + idx, vw);
+                            }
+                        }
+                    }
+                }
+            }
+            __syncwarp();  // the tables are rewritten
+            left &= ~take;
+        }
+        __syncwarp();  // the cells are rewritten
+    }
+}
+
+// The summed-area table of one stamp level per block: rows, then columns.
+__global__ void __launch_bounds__(256)
+sums_kernel(const double *stamp, int nsx, int nsy, int nx, int ny, unsigned long long *sums) {
+    const int depth = blockIdx.x;
+    const int jm = depth < 31 ? min(nsx, 1 << depth) : nsx, km = depth < 31 ? min(nsy, 1 << depth) : nsy;
+    const double *st = stamp + (long long)depth * nsx * nsy;
+    const double unit = dfrom((long long)(1023 + 62 + level_shift(jm, km, nx, ny)) << 52);
+    const long long stride = nsy + 1;
+    unsigned long long *S = sums + (long long)depth * (nsx + 1) * stride;
+    for (int j = threadIdx.x; j <= jm; j += 256) {
+        unsigned long long acc = 0;
+        S[j * stride] = 0;
+        for (int k = 0; k < km; k++) {
+            if (j > 0) acc += __double2ull_rn(ytgb::dmul(__ldg(st + (long long)(j - 1) * nsy + k), unit));
+            S[j * stride + k + 1] = acc;
+        }
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k <= km; k += 256)
+        for (int j = 1; j <= jm; j++) S[j * stride + k] += S[(j - 1) * stride + k];
+}
+
 }  // namespace
 
-extern "C" int ytgb_offaxis_cells(const ytgb_offaxis_args *args, int32_t *d_error, void *stream) {
+static int offaxis_checks(const ytgb_offaxis_args *args, const int32_t *d_error) {
     if (!args) {
         ytgb_set_error("ytgb_offaxis_cells: null args");
         return YTGB_ERR_INVALID;
@@ -368,24 +759,72 @@ extern "C" int ytgb_offaxis_cells(const ytgb_offaxis_args *args, int32_t *d_erro
         ytgb_set_error("ytgb_offaxis_cells: bad sizes (nx must not exceed ny; 2 <= max_depth <= 30)");
         return YTGB_ERR_INVALID;
     }
-    if (a.n == 0) return YTGB_OK;
-    if (!a.xp || !a.dxp || !a.qty || !a.weight || !a.stamp || !a.buffer || !a.buffer_weight ||
+    if (a.n > 0 && (!a.xp || !a.dxp || !a.qty || !a.weight || !a.stamp || !a.buffer || !a.buffer_weight ||
         ((uintptr_t)a.xp & 7) || ((uintptr_t)a.dxp & 7) || ((uintptr_t)a.qty & 7) || ((uintptr_t)a.weight & 7) ||
         ((uintptr_t)a.stamp & 7) || ((uintptr_t)a.buffer & 7) || ((uintptr_t)a.buffer_weight & 7) ||
-        ((uintptr_t)d_error & 3)) {
+        ((uintptr_t)d_error & 3))) {
         ytgb_set_error("ytgb_offaxis_cells: null or misaligned device array");
         return YTGB_ERR_INVALID;
     }
+    return YTGB_OK;
+}
+
+// Blocks for `want` warps' work, at most `per_sm` resident blocks on every SM.
+static int offaxis_blocks(long long want, int per_sm) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const long long want = (a.n + OA_WARPS - 1) / OA_WARPS;
-    const long long cap = (long long)(sms > 0 ? sms : 152) * 8;
-    const int blocks = (int)(want < cap ? want : cap);
+    const long long cap = (long long)(sms > 0 ? sms : 152) * per_sm;
+    return (int)(want < cap ? want : cap);
+}
+
+extern "C" int ytgb_offaxis_cells(const ytgb_offaxis_args *args, int32_t *d_error, void *stream) {
+    if (int st = offaxis_checks(args, d_error)) return st;
+    const ytgb_offaxis_args &a = *args;
+    if (a.n == 0) return YTGB_OK;
+    const int blocks = offaxis_blocks((a.n + OA_WARPS - 1) / OA_WARPS, 8);
     offaxis_kernel<<<blocks, OA_BLOCK, 0, (cudaStream_t)stream>>>(a, d_error);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         ytgb_set_error(std::string("ytgb_offaxis_cells: ") + cudaGetErrorString(e));
+        return YTGB_ERR_CUDA;
+    }
+    return YTGB_OK;
+}
+
+extern "C" int ytgb_offaxis_sums(const double *d_stamp, int32_t nsx, int32_t nsy, int32_t max_depth, int32_t nx,
+                                 int32_t ny, uint64_t *d_sums, void *stream) {
+    if (!d_stamp || !d_sums || ((uintptr_t)d_stamp & 7) || ((uintptr_t)d_sums & 7) || nsx < 1 || nsy < 1 ||
+        max_depth < 2 || max_depth > 30 || nx < 1 || ny < 1) {
+        ytgb_set_error("ytgb_offaxis_sums: null or misaligned array, or bad sizes");
+        return YTGB_ERR_INVALID;
+    }
+    sums_kernel<<<max_depth, 256, 0, (cudaStream_t)stream>>>(d_stamp, nsx, nsy, nx, ny,
+                                                             reinterpret_cast<unsigned long long *>(d_sums));
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) {
+        ytgb_set_error(std::string("ytgb_offaxis_sums: ") + cudaGetErrorString(e));
+        return YTGB_ERR_CUDA;
+    }
+    return YTGB_OK;
+}
+
+extern "C" int ytgb_offaxis_cells_sums(const ytgb_offaxis_args *args, const uint64_t *d_sums, int32_t *d_error,
+                                       void *stream) {
+    if (int st = offaxis_checks(args, d_error)) return st;
+    const ytgb_offaxis_args &a = *args;
+    if (!d_sums || ((uintptr_t)d_sums & 7)) {
+        ytgb_set_error("ytgb_offaxis_cells_sums: null or misaligned table of sums");
+        return YTGB_ERR_INVALID;
+    }
+    if (a.n == 0) return YTGB_OK;
+    const long long batches = (a.n + OS_CELLS - 1) / OS_CELLS;
+    const int blocks = (int)std::min<long long>((batches + OS_WARPS - 1) / OS_WARPS, 1 << 20);
+    splat_kernel<<<blocks, OS_WARPS * 32, 0, (cudaStream_t)stream>>>(
+        a, reinterpret_cast<const unsigned long long *>(d_sums), d_error);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) {
+        ytgb_set_error(std::string("ytgb_offaxis_cells_sums: ") + cudaGetErrorString(e));
         return YTGB_ERR_CUDA;
     }
     return YTGB_OK;

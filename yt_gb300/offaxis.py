@@ -11,7 +11,7 @@ spread bilinearly over the pixels it overlaps.
 :func:`offaxis_stamp` computes the stamps on the host exactly as the
 reference does (the same float64 operations, vectorised with numpy);
 :class:`CellSplat` keeps the cells resident on the device and runs the
-``ytgb_offaxis_cells`` launch; :func:`add_cells_to_image_offaxis` is the
+``ytgb_offaxis_cells_sums`` launch; :func:`add_cells_to_image_offaxis` is the
 drop-in with the reference's keyword signature, and
 :func:`project_cells` restates the driver's steps around it (recentring,
 periodic wrap, scaling by the image width, the final ``wmax / sqrt(3)``).
@@ -114,6 +114,18 @@ def _device_stamp(rotation, dx_max, nx, ny, npix_min, device):
     return torch.from_numpy(np.ascontiguousarray(eff)).to(device), stamp.shape
 
 
+def _device_sums(stamp, shape, nx, ny):
+    """The stamps' summed-area tables (``ytgb_offaxis_sums``), complete when
+    returned (a projection may run on another stream)."""
+    max_depth, nsx, nsy = shape
+    sums = torch.empty(max_depth * (nsx + 1) * (nsy + 1), dtype=torch.int64, device=stamp.device)
+    s = torch.cuda.current_stream(stamp.device)
+    _lib.check(_lib.lib().ytgb_offaxis_sums(stamp.data_ptr(), nsx, nsy, max_depth, nx, ny, sums.data_ptr(),
+                                            C.c_void_p(s.cuda_stream)), "ytgb_offaxis_sums")
+    s.synchronize()
+    return sums
+
+
 class CellSplat:
     """Cells resident on the device for repeated off-axis projections.
 
@@ -137,12 +149,15 @@ class CellSplat:
         self.weight = torch.from_numpy(weight).to(self.device)
         self.upload_bytes = 6 * 8 * self.n
         self._stamps = {}
+        self._sums = {}
 
     def stamp(self, rotation, nx, ny, npix_min=4):
         rotation = np.ascontiguousarray(rotation, dtype=np.float64).reshape(3, 3)
         key = (rotation.tobytes(), nx, ny, npix_min)
         if key not in self._stamps:
-            self._stamps[key] = _device_stamp(rotation, self.dx_max, nx, ny, npix_min, self.device)
+            stamp, shape = _device_stamp(rotation, self.dx_max, nx, ny, npix_min, self.device)
+            self._sums[key] = _device_sums(stamp, shape, nx, ny)
+            self._stamps[key] = stamp, shape
         return self._stamps[key]
 
     def project(self, rotation, nx, ny, npix_min=4, out=None, error=None, stream=None):
@@ -171,8 +186,9 @@ class CellSplat:
         a.n, a.nx, a.ny, a.nsx, a.nsy, a.max_depth = self.n, nx, ny, nsx, nsy, max_depth
         s = stream or torch.cuda.current_stream(self.device)
         err = None if error is None else error.data_ptr()
-        _lib.check(_lib.lib().ytgb_offaxis_cells(C.byref(a), C.c_void_p(err), C.c_void_p(s.cuda_stream)),
-                   "ytgb_offaxis_cells")
+        sums = self._sums[(rotation.tobytes(), nx, ny, npix_min)]
+        _lib.check(_lib.lib().ytgb_offaxis_cells_sums(C.byref(a), sums.data_ptr(), C.c_void_p(err),
+                                                      C.c_void_p(s.cuda_stream)), "ytgb_offaxis_cells_sums")
         return out
 
     def subcells(self, nx, ny, npix_min=4):
