@@ -140,3 +140,36 @@ extern "C" long long check_runs(long long n, int steps, int ties, unsigned long 
     }
     return bad;
 }
+
+#include "ytgb_octree.cuh"
+
+static double rand_t(std::mt19937_64 &g) {  // t of either sign over many binades, some with short mantissas
+    std::uniform_real_distribution<double> u(0.0, 1.0);
+    double x = std::ldexp(1.0 + u(g), (int)(g() % 40) - 30);
+    if (g() % 3 == 0) x = dfrom(dbits(x) & ~((1LL << (g() % 52)) - 1));
+    if (g() % 50 == 0) x = 0.0;
+    return x;
+}
+
+// The octree path's integer forms against float64: midpoints (positive t and
+// any t), the pair of float32 and the float32 difference; returns mismatches.
+extern "C" long long check_octree_values(long long n, unsigned long long seed) {
+    std::mt19937_64 g(seed);
+    long long bad = 0;
+    for (long long k = 0; k < n; k++) {
+        const double a = rand_t(g), b = g() % 2 ? a * (1.0 + 1e-3 * (double)(g() % 1000)) : rand_t(g);
+        const double mid = (a + b) * 0.5;
+        if (dbits(midpoint<T_BITS>(a, b)) != dbits(mid) || dbits(midpoint<T_KEYS>(a, b)) != dbits(mid)) bad++;
+        const double c = g() % 2 ? -b : b, m2 = (a + c) * 0.5;
+        const double got = midpoint<T_KEYS>(a, c);
+        if (!(got == m2)) bad++;
+        float hi, lo;
+        split_pair(c, hi, lo);
+        const float fh = (float)c;
+        const bool tie = std::fabs(c - (double)fh) == std::fabs((double)std::nextafter(fh, c > (double)fh ? INFINITY : -INFINITY) - c);
+        if (!tie && (hi != fh || lo != (float)(c - (double)fh))) bad++;
+        if (tie && (double)hi + (double)lo != c) bad++;
+        if (diff_nearest(b, a) != (float)(b - a)) bad++;
+    }
+    return bad;
+}

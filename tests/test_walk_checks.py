@@ -46,3 +46,11 @@ def test_runs_of_steps_equal_float64_adds(checks, steps, ties):
     bad = checks.check_runs(C.c_longlong(n), steps, ties, C.c_ulonglong(5 + steps), C.byref(looks))
     assert bad == 0
     assert looks.value > 0
+
+
+def test_octree_values_equal_float64(checks):
+    """Slab midpoints, float32 pairs and dt formed on the integer pipe are the
+    float64 operations' (float32 ties, which the pair rounds the other way,
+    still sum to the value)."""
+    checks.check_octree_values.restype = C.c_longlong
+    assert checks.check_octree_values(C.c_longlong(2_000_000), C.c_ulonglong(3)) == 0

@@ -1285,9 +1285,11 @@ YTGB_HD float approx_float(long long x) {
 #ifdef __CUDA_ARCH__
 YTGB_HD unsigned walking_lanes() { return __activemask(); }
 YTGB_HD void meet(unsigned lanes) { __syncwarp(lanes); }
+YTGB_HD bool any_lane(unsigned lanes, bool p) { return __any_sync(lanes, p); }
 #else
 YTGB_HD unsigned walking_lanes() { return 0; }
 YTGB_HD void meet(unsigned) {}
+YTGB_HD bool any_lane(unsigned, bool p) { return p; }
 #endif
 
 // One axis of a run of steps: how far tmax (float64 bits x, below max_t)
