@@ -388,7 +388,8 @@ int tf_check(const ytgb_tf &t, size_t *smem, bool ctf_layout) {
 
 template <typename K>
 int set_smem(K kernel, size_t smem) {
-    if (smem > 48 * 1024) {
+    // (static and dynamic shared memory together need the opt-in past 48 KB)
+    if (smem + sizeof(TileSmem) > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) {
             ytgb_set_error(std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
