@@ -793,15 +793,7 @@ YTGB_HD bool range_ambiguous(float v, float tol, float lo, float hi) {
 // fields.  Where the field is exactly flat the reference normalises its
 // rounding noise into an arbitrary direction; here the gradient is 0.  A
 // NaN corner (log10 of a non-positive vertex value) makes the gradient NaN.
-YTGB_HD void light_gradient(const float *__restrict__ p, const float *__restrict__ lo, int sy, int sx, float dx,
-                            float dy, float dz, float g[3]) {
-    float c[8], e[8];
-    YTGB_UNROLL
-    for (int q = 0; q < 8; q++) {
-        const int o = ((q >> 2) & 1) * sx + ((q >> 1) & 1) * sy + (q & 1);
-        c[q] = ldg(p + o);
-        e[q] = lo ? ldg(lo + o) : 0.0f;
-    }
+YTGB_HD void light_gradient(const float c[8], const float e[8], float dx, float dy, float dz, float g[3]) {
     // corner q = 4a + 2b + c at offsets a (x), b (y), c (z)
 #define YTGB_D(u, v) fadd(fsub(c[u], c[v]), fsub(e[u], e[v]))
     const float x00 = YTGB_D(4, 0), x01 = YTGB_D(5, 1), x10 = YTGB_D(6, 2), x11 = YTGB_D(7, 3);
@@ -827,6 +819,11 @@ YTGB_HD void light_gradient(const float *__restrict__ p, const float *__restrict
         // is every channel it composites (0 * NaN), as here
         g[0] = g[1] = g[2] = __builtin_nanf("");
     }
+}
+
+YTGB_HD void load_corners(const float *__restrict__ p, int sy, int sx, float c[8]) {
+    YTGB_UNROLL
+    for (int q = 0; q < 8; q++) c[q] = ldg(p + ((q >> 2) & 1) * sx + ((q >> 1) & 1) * sy + (q & 1));
 }
 
 // One bin of the packed ColorTransferFunction tables: the four tables' y and
@@ -984,6 +981,19 @@ struct CellCtx {
 // range_eps > 0).
 constexpr int V_CTF = 1;
 constexpr int V_REF = 2;
+// The single-view kernel only (not part of a launch's variant): compiled with
+// sample_many.  Kept out of the others, whose simple loop it slows (more state
+// across one kernel: the AMR frame 1.36 -> 1.43 ms, 16 views in a batch 4.5 ->
+// 5.1 ms).  The batch kernel takes such walks through the loop with every test
+// in every step: with sample_many inlined for the light source or other table
+// sets, a build of it at 128 registers met an illegal address whose cause
+// reading did not show.
+constexpr int V_MANY = 4;
+#ifdef __CUDACC__
+constexpr bool MANY_ALWAYS = false;
+#else
+constexpr bool MANY_ALWAYS = true;  // the test harness takes every walk through it
+#endif
 
 // The variant a render's arguments call for: float64 range decisions where
 // the arena's rounding errors and their scale are given, except for a
@@ -1029,10 +1039,11 @@ YTGB_HD float cell_coord(float x) {
     return CLAMP ? fminf(fmaxf(x, 0.0f), 1.0f) : x;
 }
 
-template <int MODE, int VAR, bool CLAMP = true, bool TG = false>
+// COUNT: whether it counts the visit (the fast cell loop counts its own).
+template <int MODE, int VAR, bool CLAMP = true, bool TG = false, bool COUNT = true>
 YTGB_HD void sample_cell(const ytgb_render_args &a, const float4 *s_tab, int bi, const CellCtx &c, const int cur[3],
                          const float P[3], float dtf, long long enter_bits, long long exit_bits, RayState &st) {
-    st.visits++;
+    if (COUNT) st.visits++;
     if (MODE == MODE_TRACE) {
         st.th = fnv_mix(st.th, (unsigned long long)(unsigned)bi);
         st.th = fnv_mix(st.th, (unsigned long long)(unsigned)cur[0] | ((unsigned long long)(unsigned)cur[1] << 32));
@@ -1068,8 +1079,10 @@ YTGB_HD void sample_cell(const ytgb_render_args &a, const float4 *s_tab, int bi,
             YTGB_UNROLL
             for (int fi = 0; fi < 6; fi++)
                 if (fi < c.nf) dvs[fi] = trilinear(c.base + fi * c.fstride + off, c.sy, c.sx, fx, fy, fz);
-            float g[3];
-            light_gradient(c.base + off, lo, c.sy, c.sx, fx, fy, fz, g);
+            float g[3], cv[8], ce[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            load_corners(c.base + off, c.sy, c.sx, cv);
+            if (lo) load_corners(lo, c.sy, c.sx, ce);
+            light_gradient(cv, ce, fx, fy, fz, g);
             const float dot = ffma(a.light_dir[2], g[2], ffma(a.light_dir[1], g[1], fmul(a.light_dir[0], g[0])));
             float trgba[6];
             unsigned force = 0u, force_in = 0u;
@@ -1371,15 +1384,23 @@ YTGB_HD F2 fma2(F2 a, F2 b, F2 c) { return {std::fmaf(a.x, b.x, c.x), std::fmaf(
 #endif
 YTGB_HD F2 sub2(F2 a, F2 b) { return fma2(b, f2(-1.0f, -1.0f), a); }  // (a + -1 b: one rounding, as a - b)
 
-// trilinear, its lerps along z and y two at a time
-YTGB_HD float trilinear2(const float *__restrict__ p, int sy, int sx, float dx, float dy, float dz) {
-    const F2 l0 = f2(ldg(p), ldg(p + sx)), u0 = f2(ldg(p + 1), ldg(p + sx + 1));
-    const F2 l1 = f2(ldg(p + sy), ldg(p + sx + sy)), u1 = f2(ldg(p + sy + 1), ldg(p + sx + sy + 1));
+// trilinear, its lerps along z and y two at a time, from the cell's corners
+// (q = 4a + 2b + c at offsets a (x), b (y), c (z)) or from memory (pair by pair:
+// in the corners' order the AMR frame and projection run 1 and 3 % slower)
+YTGB_HD float lerp_pairs(F2 l0, F2 u0, F2 l1, F2 u1, float dx, float dy, float dz) {
     const F2 z = f2(dz, dz), y = f2(dy, dy);
     const F2 a0 = fma2(z, sub2(u0, l0), l0);  // a0, a2
     const F2 a1 = fma2(z, sub2(u1, l1), l1);  // a1, a3
     const F2 b = fma2(y, sub2(a1, a0), a0);
     return ffma(dx, fsub(f2y(b), f2x(b)), f2x(b));
+}
+YTGB_HD float trilinear2(const float q[8], float dx, float dy, float dz) {
+    return lerp_pairs(f2(q[0], q[4]), f2(q[1], q[5]), f2(q[2], q[6]), f2(q[3], q[7]), dx, dy, dz);
+}
+YTGB_HD float trilinear2(const float *__restrict__ p, int sy, int sx, float dx, float dy, float dz) {
+    const F2 l0 = f2(ldg(p), ldg(p + sx)), u0 = f2(ldg(p + 1), ldg(p + sx + 1));
+    const F2 l1 = f2(ldg(p + sy), ldg(p + sx + sy)), u1 = f2(ldg(p + sy + 1), ldg(p + sx + sy + 1));
+    return lerp_pairs(l0, u0, l1, u1, dx, dy, dz);
 }
 
 // emit_sel of two channels
@@ -1400,6 +1421,78 @@ YTGB_HD void emit_sel2(float &h0, float &l0, float &h1, float &l1, F2 d) {
     l0 = a ? f2x(l) : 0.0f;
     h1 = b ? f2y(h) : f2y(d);
     l1 = b ? f2y(l) : 0.0f;
+}
+
+// acc_grey of two channels, where the sample is in range
+template <bool COMP>
+YTGB_HD void grey_sel2(float &h0, float &l0, float &h1, float &l1, float dt, F2 e, float da, bool in) {
+    const F2 h = f2(h0, h1), l = f2(l0, l1), t = f2(dt, dt), a = f2(da, da);
+    const F2 de = mul2(t, e);
+    F2 s, r = l;
+    if (COMP) {
+        const F2 p = mul2(a, h);
+        const F2 de_l = fma2(t, e, mul2(f2(-dt, -dt), e));      // dt e - de
+        const F2 p_l = fma2(a, h, mul2(f2(-da, -da), h));       // da x - p
+        const F2 inc = sub2(add2(sub2(de, p), sub2(de_l, p_l)), mul2(a, l));
+        s = add2(h, inc);
+        const F2 bp = sub2(s, h);
+        r = add2(l, add2(sub2(h, sub2(s, bp)), sub2(inc, bp)));
+    } else {
+        s = fma2(f2(-da, -da), h, add2(h, de));
+    }
+    const bool small = da < 1.0f;
+    h0 = in ? (small ? f2x(s) : f2x(de)) : h0;
+    h1 = in ? (small ? f2y(s) : f2y(de)) : h1;
+    l0 = in ? (small ? f2x(r) : 0.0f) : l0;
+    l1 = in ? (small ? f2y(r) : 0.0f) : l1;
+}
+
+// The three channels' emission times alpha of a ColorTransferFunction from its
+// tables as ytgb_tf_pack lays them out (in global or shared memory).
+YTGB_HD void ctf_emission(const ytgb_tf &tf, const float4 *tab, float val, float e[3]) {
+    float q = fmul(fsub(val, tf.b0[0]), tf.idbin[0]);
+    q = fminf(fmaxf(q, 0.0f), (float)(tf.nbins[0] - 2));
+    const float4 *t = tab + (int)q;
+    const float4 t3 = t[3 * tf.nbins_max];
+    const float dd = fsub(fsub(val, t3.z), t3.w);
+    const float al = ffma(dd, t3.y, t3.x);
+    YTGB_UNROLL
+    for (int ch = 0; ch < 3; ch++) {
+        const float4 v = t[ch * tf.nbins_max];
+        e[ch] = fmul(ffma(dd, v.y, v.x), al);
+    }
+}
+
+// FIT_get_value's range test of a ColorTransferFunction in float32 (NaN and
+// infinities fail the strict bound tests, so they need no separate test)
+YTGB_HD bool ctf_in(const ytgb_tf &tf, float val) { return val < tf.hi_excl[0] && val > tf.lo_excl[0] && val != 0.0f; }
+
+// A sample value through the ColorTransferFunction tables into the image; the
+// range test (in) and the update are selects.
+template <bool COMP, bool TG>
+YTGB_HD void shade_ctf(const ytgb_tf &tf, const float4 *s_tab, float val, bool in, bool grey, float dtf,
+                       RayState &st) {
+    float q = fmul(fsub(val, tf.b0[0]), tf.idbin[0]);
+    q = fminf(fmaxf(q, 0.0f), (float)(tf.nbins[0] - 2));  // a NaN q gives bin 0 (the sample is then out of range)
+    const int bin = (int)q;
+    float4 Y, D;
+    float2 Z;
+    ctf_bin<TG>(s_tab, tf.nbins_max, bin, Y, D, Z);
+    const float dd = fsub(fsub(val, Z.x), Z.y);
+    const F2 dd2 = f2(dd, dd);
+    const F2 e01 = fma2(dd2, f2(D.x, D.y), f2(Y.x, Y.y)), e23 = fma2(dd2, f2(D.z, D.w), f2(Y.z, Y.w));
+    const float al = f2y(e23);
+    const F2 erg = mul2(e01, f2(al, al));
+    const float eb_ = fmul(f2x(e23), al);
+    if (grey) {
+        const float da = fmul(dtf, al);
+        grey_sel2<COMP>(st.xh[0], st.xl[0], st.xh[1], st.xl[1], dtf, erg, da, in);
+        grey_sel2<COMP>(st.xh[2], st.xl[2], st.xh[3], st.xl[3], dtf, f2(eb_, al), da, in);
+    } else {
+        const F2 d = mul2(f2(dtf, dtf), erg);
+        emit_sel2<COMP>(st.xh[0], st.xl[0], st.xh[1], st.xl[1], f2(in ? f2x(d) : 0.0f, in ? f2y(d) : 0.0f));
+        emit_sel<COMP>(st.xh[2], st.xl[2], in ? fmul(dtf, eb_) : 0.0f);
+    }
 }
 
 // One sample of the fast cell loop (n_samples = 1): the value at the middle
@@ -1441,45 +1534,96 @@ YTGB_HD void sample_fast(const ytgb_render_args &a, const float4 *s_tab, const R
         return;
     }
     if (!(MODE == MODE_VR && (VAR & V_CTF))) return;
-    const ytgb_tf &tf = a.tf;
-    const bool grey = GREY >= 0 ? GREY == 1 : tf.grey_opacity == 1;
     const float val = trilinear2(c.base + off, c.sy, c.sx, fx, fy, fz);
-    // (NaN and infinities fail the strict bound tests, so they need no separate test)
-    bool in = val < tf.hi_excl[0] && val > tf.lo_excl[0] && val != 0.0f;
-    if ((VAR & V_REF) && range_ambiguous(val, c.tol, tf.lo_excl[0], tf.hi_excl[0])) {
+    bool in = ctf_in(a.tf, val);
+    if ((VAR & V_REF) && range_ambiguous(val, c.tol, a.tf.lo_excl[0], a.tf.hi_excl[0])) {
         // decide as yt does, from the float64 value (rare)
-        in = range_in64(&r, bp, c.base + off, a.data_lo + (c.base - a.data) + off, c.sy, c.sx, c0, c1, c2, eb,
-                        xb, 1, 0, tf.bound64[0][0], tf.bound64[0][1]);
+        in = range_in64(&r, bp, c.base + off, a.data_lo + (c.base - a.data) + off, c.sy, c.sx, c0, c1, c2, eb, xb, 1,
+                        0, a.tf.bound64[0][0], a.tf.bound64[0][1]);
     }
-    float q = fmul(fsub(val, tf.b0[0]), tf.idbin[0]);
-    q = fminf(fmaxf(q, 0.0f), (float)(tf.nbins[0] - 2));  // a NaN q gives bin 0 (the sample is then out of range)
-    const int bin = (int)q;
-    float4 Y, D;
-    float2 Z;
-    ctf_bin<TG>(s_tab, tf.nbins_max, bin, Y, D, Z);
-    const float dd = fsub(fsub(val, Z.x), Z.y);
-    const F2 dd2 = f2(dd, dd);
-    const F2 e01 = fma2(dd2, f2(D.x, D.y), f2(Y.x, Y.y)), e23 = fma2(dd2, f2(D.z, D.w), f2(Y.z, Y.w));
-    const float al = f2y(e23);
-    const F2 erg = mul2(e01, f2(al, al));
-    const float er = f2x(erg), eg = f2y(erg), eb_ = fmul(f2x(e23), al);
-    if (grey) {
-        float h[4] = {st.xh[0], st.xh[1], st.xh[2], st.xh[3]};
-        float l[4] = {st.xl[0], st.xl[1], st.xl[2], st.xl[3]};
-        const float da = fmul(dtf, al);
-        acc_grey(h[0], l[0], dtf, er, da, COMP);
-        acc_grey(h[1], l[1], dtf, eg, da, COMP);
-        acc_grey(h[2], l[2], dtf, eb_, da, COMP);
-        acc_grey(h[3], l[3], dtf, al, da, COMP);
+    shade_ctf<COMP, TG>(a.tf, s_tab, val, in, GREY >= 0 ? GREY == 1 : a.tf.grey_opacity == 1, dtf, st);
+}
+
+// The samples of one cell for the walks that are not the fast loop's simplest:
+// several samples per cell, masked bricks, the light source, other table sets.
+// A cell's corners are loaded once for all its samples, the range test and the
+// update are selects, and a light source's ColorTransferFunction is one bin
+// look-up (as six general tables its registers spilled).  The same values as
+// sample_cell's, which takes the table sets that have no form here.  Issue-bound
+// (57 %, 24 of 32 lanes).  Kernel times against sample_cell in the loop with its
+// tests in every step: ten samples per cell 640x480 2.27 -> 1.10 ms, light
+// source 512^2 1.80 -> 0.61, three samples of a 1024x768 interpolated projection
+// 2.50 -> 1.75, three general tables 701x1003 1.47 -> 1.14.
+template <int MODE, int VAR, bool COMP, bool TG>
+YTGB_HD void sample_many(const ytgb_render_args &a, const float4 *s_tab, const Ray &r, const ytgb_brick *bp,
+                         const CellCtx &c, int c0, int c1, int c2, float P0, float P1, float P2, float dtf,
+                         long long eb, long long xb, RayState &st) {
+    const int ns = a.n_samples;
+    const bool ctf = MODE == MODE_VR ? (VAR & V_CTF) != 0 : MODE == MODE_LIGHT && a.tf.ctf_fast != 0;
+    if (MODE != MODE_IPROJ && !ctf) {
+        const int cur[3] = {c0, c1, c2};
+        const float P[3] = {P0, P1, P2};
+        sample_cell<MODE, VAR, true, TG, false>(a, s_tab, 0, c, cur, P, dtf, eb, xb, st);
+        return;
+    }
+    const int off = c0 * c.sx + c1 * c.sy + c2;
+    const float dts = ns == 1 ? dtf : fdiv(dtf, (float)ns);
+    if (MODE == MODE_IPROJ) {
+        const int n3 = c.nf < 3 ? c.nf : 3;
+        st.touched |= (1u << n3) - 1u;
         YTGB_UNROLL
-        for (int ch = 0; ch < 4; ch++) {
-            st.xh[ch] = in ? h[ch] : st.xh[ch];
-            st.xl[ch] = in ? l[ch] : st.xl[ch];
+        for (int ch = 0; ch < 3; ch++) {
+            if (ch < n3) {
+                float q[8];
+                load_corners(c.base + ch * c.fstride + off, c.sy, c.sx, q);
+                for (int s = 0; s < ns; s++) {
+                    const float f = fmul(dts, (float)s + 0.5f);
+                    const float v = trilinear2(q, ffma_sat(f, c.vel[0], P0), ffma_sat(f, c.vel[1], P1),
+                                               ffma_sat(f, c.vel[2], P2));
+                    add_sel<COMP>(st.xh[ch], st.xl[ch], fmul(v, dts));
+                }
+            }
         }
-    } else {
-        const F2 d = mul2(f2(dtf, dtf), erg);
-        emit_sel2<COMP>(st.xh[0], st.xl[0], st.xh[1], st.xl[1], f2(in ? f2x(d) : 0.0f, in ? f2y(d) : 0.0f));
-        emit_sel<COMP>(st.xh[2], st.xl[2], in ? fmul(dtf, eb_) : 0.0f);
+        return;
+    }
+    if (MODE == MODE_VR && c.moff >= 0 && a.masks &&
+        ldg(a.masks + c.moff + (c0 * c.dims[1] + c1) * c.dims[2] + c2) != 1)
+        return;
+    const float *lo = a.data_lo ? a.data_lo + (c.base - a.data) + off : nullptr;
+    const bool grey = a.tf.grey_opacity == 1;
+    st.touched |= MODE == MODE_VR && grey ? 0xfu : 0x7u;
+    float q[8], ce[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    load_corners(c.base + off, c.sy, c.sx, q);
+    if (MODE == MODE_LIGHT && lo) load_corners(lo, c.sy, c.sx, ce);
+    for (int s = 0; s < ns; s++) {
+        const float f = fmul(dts, (float)s + 0.5f);
+        const float fx = ffma_sat(f, c.vel[0], P0), fy = ffma_sat(f, c.vel[1], P1), fz = ffma_sat(f, c.vel[2], P2);
+        const float val = trilinear2(q, fx, fy, fz);
+        bool in = ctf_in(a.tf, val);
+        if ((VAR & V_REF) && c.tol >= 0.0f && a.tf.lo_excl[0] <= a.tf.hi_excl[0] &&
+            range_ambiguous(val, c.tol, a.tf.lo_excl[0], a.tf.hi_excl[0])) {
+            // decide as yt does, from the float64 value (rare)
+            in = range_in64(&r, bp, c.base + off, lo, c.sy, c.sx, c0, c1, c2, eb, xb, ns, s, a.tf.bound64[0][0],
+                            a.tf.bound64[0][1]);
+        }
+        if (MODE == MODE_VR) {
+            shade_ctf<COMP, TG>(a.tf, s_tab, val, in, grey, dts, st);
+        } else {
+            // LightSourceRenderSampler.sample, as in sample_cell: zero emission
+            // out of range, so that a NaN gradient still reaches the image
+            float g[3];
+            light_gradient(q, ce, fx, fy, fz, g);
+            const float dot = ffma(a.light_dir[2], g[2], ffma(a.light_dir[1], g[1], fmul(a.light_dir[0], g[0])));
+            float e[3];
+            ctf_emission(a.tf, s_tab, val, e);
+            YTGB_UNROLL
+            for (int ch = 0; ch < 3; ch++) e[ch] = in ? e[ch] : 0.0f;
+            const float dg = fmul(dts, fadd(fadd(e[0], e[1]), e[2]));
+            YTGB_UNROLL
+            for (int ch = 0; ch < 3; ch++)
+                acc_light(st.xh[ch], st.xl[ch], grey ? dg : fmul(dts, e[ch]),
+                          fmul(e[ch], ffma(dot, a.light_rgba[ch], 1.0f)), COMP);
+        }
     }
 }
 
@@ -1509,12 +1653,14 @@ YTGB_HD void sample_fast(const ytgb_render_args &a, const float4 *s_tab, const R
 // other, 34.6 ms for that projection; the walk's last cell inside the loop,
 // 7 % slower on the AMR frame; adds on the multiply pipe (mad.wide), 9 %
 // slower on the projection.
+// MANY: the cell's samples by sample_many, whose code is not repeated for the
+// walk's last cell (taken inside the loop).
 // NCH: the channels the projection samplers write, when the launch fixes
 // it (1: one field, the common case); 0 reads it from the brick.  A runtime
 // channel count leaves every channel's instructions in the loop, predicated
 // off but still issued (one field: the projection 24 % and the MIP 27 %
 // faster with NCH = 1).  GREY: grey_opacity fixed (0 or 1) or read (-1).
-template <int MODE, int VAR, bool COMP, bool TG, int NCH = 0, int GREY = -1>
+template <int MODE, int VAR, bool COMP, bool TG, int NCH = 0, int GREY = -1, bool MANY = false>
 YTGB_HD void cells_fast(const ytgb_render_args &a, const float4 *s_tab, Ray &r, const ytgb_brick *bp,
                         const CellCtx &c, const Walk &w, long long kmax, int step_limit, RayState &st) {
     long long T0 = dbits(w.tmax[0]), T1 = dbits(w.tmax[1]), T2 = dbits(w.tmax[2]);
@@ -1566,18 +1712,22 @@ YTGB_HD void cells_fast(const ytgb_render_args &a, const float4 *s_tab, Ray &r, 
         tmb = s2 ? T2 : tmb;
         const bool look = tmb >= lim;
         float dtl = 0.0f;
+        bool last = false;
         if (__builtin_expect(look, 0)) {
             const int i = s0 ? 0 : (s1 ? 1 : 2);
             const int ci = s0 ? c0 : (s1 ? c1 : c2), di = s0 ? d0 : (s1 ? d1 : d2);
             const int dn = s0 ? c.dims[0] : (s1 ? c.dims[1] : c.dims[2]);
             // the stepped index leaves the brick, or exit_t >= max_t
-            if ((unsigned)(ci + di) >= (unsigned)dn || !(tmb < kmax)) break;
+            last = (unsigned)(ci + di) >= (unsigned)dn || !(tmb < kmax);
             if (++looks > step_limit) {
                 set_error(a.error, YTGB_DEVERR_STEP_LIMIT);
-                break;
+                last = true;
             }
-            if (DT) dtl = diff_to_float_loop(tmb, eb);
-            if (tmb >= r.lim[i]) {
+            if (!MANY && last) break;
+            if (MANY && last)
+                st.visits += (unsigned)((c0 - w.cur[0]) * d0 + (c1 - w.cur[1]) * d1 + (c2 - w.cur[2]) * d2) + 1u;
+            if (DT) dtl = diff_to_float_loop(MANY && kmax < tmb ? kmax : tmb, eb);
+            if (!last && tmb >= r.lim[i]) {
                 // (the ray is in shared memory: a runtime index costs no local memory)
                 const double td = r.td[i];
                 const long long nb = dbits(dadd(dfrom(tmb), td));
@@ -1610,8 +1760,12 @@ YTGB_HD void cells_fast(const ytgb_render_args &a, const float4 *s_tab, Ray &r, 
             dtf = fmul(approx_float(tmb - eb), scale);
             dtf = look ? dtl : dtf;
         }
-        sample_fast<MODE, VAR, COMP, TG, NCH, GREY>(a, s_tab, r, bp, c, c0, c1, c2, P0, P1, P2, dtf, eb, tmb,
-                                                    st);
+        if (MANY)
+            sample_many<MODE, VAR, COMP, TG>(a, s_tab, r, bp, c, c0, c1, c2, P0, P1, P2, dtf, eb,
+                                             kmax < tmb ? kmax : tmb, st);
+        else
+            sample_fast<MODE, VAR, COMP, TG, NCH, GREY>(a, s_tab, r, bp, c, c0, c1, c2, P0, P1, P2, dtf, eb, tmb,
+                                                        st);
         // advance (grid_traversal.pyx:134-138): the position to the exit
         // point, the stepped axis onto the next cell's entry face
         if (!CELLS) {
@@ -1623,16 +1777,19 @@ YTGB_HD void cells_fast(const ytgb_render_args &a, const float4 *s_tab, Ray &r, 
         add_where(s1, T1, I1, c1, d1);
         add_where(s2, T2, I2, c2, d2);
         eb = tmb;
+        if (MANY && last) break;
     }
     meet(lanes);
-    // the walk's last cell
-    const long long xb = tmb < kmax ? tmb : kmax;  // fmin(tmax[i], max_t)
-    const float dtf = DT ? diff_to_float_loop(xb, eb) : 0.0f;
-    sample_fast<MODE, VAR, COMP, TG, NCH, GREY>(a, s_tab, r, bp, c, c0, c1, c2, P0, P1, P2, dtf, eb, xb, st);
-    st.visits += (unsigned)((c0 - w.cur[0]) * d0 + (c1 - w.cur[1]) * d1 + (c2 - w.cur[2]) * d2) + 1u;
-    if (MODE == MODE_VR) st.touched |= a.tf.grey_opacity == 1 ? 0xfu : 0x7u;
-    else if (MODE == MODE_IPROJ) st.touched |= (1u << (c.nf < 3 ? c.nf : 3)) - 1u;
-    else st.touched |= (1u << (c.nf < 4 ? c.nf : 4)) - 1u;
+    if (!MANY) {
+        // the walk's last cell
+        const long long xb = tmb < kmax ? tmb : kmax;  // fmin(tmax[i], max_t)
+        const float dtf = DT ? diff_to_float_loop(xb, eb) : 0.0f;
+        sample_fast<MODE, VAR, COMP, TG, NCH, GREY>(a, s_tab, r, bp, c, c0, c1, c2, P0, P1, P2, dtf, eb, xb, st);
+        st.visits += (unsigned)((c0 - w.cur[0]) * d0 + (c1 - w.cur[1]) * d1 + (c2 - w.cur[2]) * d2) + 1u;
+        if (MODE == MODE_VR) st.touched |= a.tf.grey_opacity == 1 ? 0xfu : 0x7u;
+        else if (MODE == MODE_IPROJ) st.touched |= (1u << (c.nf < 3 ? c.nf : 3)) - 1u;
+        else st.touched |= (1u << (c.nf < 4 ? c.nf : 4)) - 1u;
+    }
 }
 
 // One brick of one ray: cast_through_kdtree's walk_volume call
@@ -1680,20 +1837,32 @@ YTGB_HD void walk_brick(const ytgb_render_args &a, const float4 *s_tab, Ray &r, 
     const long long b0 = dbits(w.tmax[0]), b1 = dbits(w.tmax[1]), b2 = dbits(w.tmax[2]);
     const long long INF = 0x7ff0000000000000LL;
     const bool int_path = b0 > 0 && b1 > 0 && b2 > 0 && b0 < INF && b1 < INF && b2 < INF && kmax > 0;
-    if (MODE != MODE_TRACE && MODE != MODE_LIGHT && (MODE != MODE_VR || (VAR & V_CTF)) && int_path && a.n_samples == 1 &&
-        (MODE != MODE_VR || c.moff < 0 || !a.masks) && (unsigned)w.cur[0] < (unsigned)c.dims[0] &&
+    if (MODE != MODE_TRACE && int_path && (unsigned)w.cur[0] < (unsigned)c.dims[0] &&
         (unsigned)w.cur[1] < (unsigned)c.dims[1] && (unsigned)w.cur[2] < (unsigned)c.dims[2]) {
-        if (MODE != MODE_VR && c.nf == 1) {
-            if (st.comp) cells_fast<MODE, VAR, true, TG, 1>(a, s_tab, r, bp, c, w, kmax, step_limit, st);
-            else cells_fast<MODE, VAR, false, TG, 1>(a, s_tab, r, bp, c, w, kmax, step_limit, st);
-        } else if (MODE == MODE_VR && a.tf.grey_opacity != 1) {
-            if (st.comp) cells_fast<MODE, VAR, true, TG, 0, 0>(a, s_tab, r, bp, c, w, kmax, step_limit, st);
-            else cells_fast<MODE, VAR, false, TG, 0, 0>(a, s_tab, r, bp, c, w, kmax, step_limit, st);
-        } else {
-            if (st.comp) cells_fast<MODE, VAR, true, TG>(a, s_tab, r, bp, c, w, kmax, step_limit, st);
-            else cells_fast<MODE, VAR, false, TG>(a, s_tab, r, bp, c, w, kmax, step_limit, st);
+        // one sample per cell (the cell samplers take no other number), no mask
+        // and a form of its own for the table set: sample_fast; else sample_many
+        const bool simple = MODE == MODE_PROJ || MODE == MODE_MIP ||
+                            ((MODE == MODE_IPROJ || (MODE == MODE_VR && (VAR & V_CTF))) && a.n_samples == 1 &&
+                             (MODE != MODE_VR || c.moff < 0 || !a.masks));
+        constexpr bool MANY = (VAR & V_MANY) != 0 || MANY_ALWAYS;
+        if (MANY && !simple) {
+            if (st.comp) cells_fast<MODE, VAR, true, TG, 0, -1, true>(a, s_tab, r, bp, c, w, kmax, step_limit, st);
+            else cells_fast<MODE, VAR, false, TG, 0, -1, true>(a, s_tab, r, bp, c, w, kmax, step_limit, st);
+            return;
         }
-        return;
+        if (simple) {
+            if (MODE != MODE_VR && c.nf == 1) {
+                if (st.comp) cells_fast<MODE, VAR, true, TG, 1>(a, s_tab, r, bp, c, w, kmax, step_limit, st);
+                else cells_fast<MODE, VAR, false, TG, 1>(a, s_tab, r, bp, c, w, kmax, step_limit, st);
+            } else if (MODE == MODE_VR && a.tf.grey_opacity != 1) {
+                if (st.comp) cells_fast<MODE, VAR, true, TG, 0, 0>(a, s_tab, r, bp, c, w, kmax, step_limit, st);
+                else cells_fast<MODE, VAR, false, TG, 0, 0>(a, s_tab, r, bp, c, w, kmax, step_limit, st);
+            } else {
+                if (st.comp) cells_fast<MODE, VAR, true, TG>(a, s_tab, r, bp, c, w, kmax, step_limit, st);
+                else cells_fast<MODE, VAR, false, TG>(a, s_tab, r, bp, c, w, kmax, step_limit, st);
+            }
+            return;
+        }
     }
     // tdelta = step * iv_dir * dds (grid_traversal.pyx:86)
     double tdelta[3];

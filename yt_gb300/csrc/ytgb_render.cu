@@ -78,8 +78,13 @@ constexpr int NWARP = BLOCK / 32;
 //   ColorTransferFunction rendering: 5, 96 registers: 1.362 ms on the 1024^2
 //     AMR frame (6: 1.406);
 //   with float64 range decisions (V_REF), whose rare path needs the most: 4,
-//     128 registers: 505 us on a 701x1003 AMR frame (5: 545);
-//   other table sets, the light source and the traversal trace: 6.
+//     128 registers: 500 us on a 701x1003 AMR frame (5: 545);
+//   with sample_many (V_MANY, the light source, other table sets): 4, where the
+//     corners stay in registers over a cell's samples: ten samples per cell
+//     640x480 1.10 ms (5: 1.33, 6: 1.67), light source 512^2 0.61 (5: 0.76, 6:
+//     1.00), three tables 701x1003 1.14 (5: 1.30, 6: 1.60); interpolated
+//     projection 6;
+//   the traversal trace: 6.
 // The persistent batch kernel, whose loop keeps more state: 5 (4.56 ms for 16
 // views; 4: 4.66, 6: 4.80).  Images are identical at every setting.
 // YTGB_MIN_BLOCKS sets all (a second build at another budget, for the
@@ -89,10 +94,11 @@ constexpr int min_blocks(int, int) { return YTGB_MIN_BLOCKS; }
 constexpr int BATCH_MIN_BLOCKS = YTGB_MIN_BLOCKS;
 #else
 constexpr int min_blocks(int mode, int var) {
-    return (var & V_REF) ? 4
-           : mode == MODE_PROJ || mode == MODE_MIP ? 7
-           : mode == MODE_VR && (var & V_CTF) ? 5
-                                              : 6;
+    return mode == MODE_PROJ || mode == MODE_MIP ? 7
+           : mode == MODE_IPROJ                  ? 6
+           : (var & (V_REF | V_MANY))            ? 4
+           : (var & V_CTF)                       ? 5
+                                                 : 6;
 }
 constexpr int BATCH_MIN_BLOCKS = 5;
 #endif
@@ -434,13 +440,20 @@ int launch_ts(int ts, const ytgb_render_args *a, size_t smem, cudaStream_t s, un
 
 int tile_shape_of(uint32_t flags) { return (int)((flags >> YTGB_FLAG_TILE_SHIFT) & 0xfu); }
 
-template <int MODE>
-int launch_var(int var, int ts, const ytgb_render_args *a, size_t smem, cudaStream_t s) {
+// Volume rendering: the launch's variant, with sample_many where the
+// ColorTransferFunction walks are not all of one sample per unmasked cell
+// (other table sets have no simpler form).
+int launch_vr(int var, int ts, const ytgb_render_args *a, size_t smem, cudaStream_t s) {
+    const bool many = a->n_samples != 1 || a->masks;
     switch (var) {
-    case V_CTF: return launch_ts<MODE, V_CTF>(ts, a, smem, s, nullptr, nullptr);
-    case V_REF: return launch_ts<MODE, V_REF>(ts, a, smem, s, nullptr, nullptr);
-    case V_CTF | V_REF: return launch_ts<MODE, V_CTF | V_REF>(ts, a, smem, s, nullptr, nullptr);
-    default: return launch_ts<MODE, 0>(ts, a, smem, s, nullptr, nullptr);
+    case V_CTF:
+        return many ? launch_ts<MODE_VR, V_CTF | V_MANY>(ts, a, smem, s, nullptr, nullptr)
+                    : launch_ts<MODE_VR, V_CTF>(ts, a, smem, s, nullptr, nullptr);
+    case V_REF: return launch_ts<MODE_VR, V_REF | V_MANY>(ts, a, smem, s, nullptr, nullptr);
+    case V_CTF | V_REF:
+        return many ? launch_ts<MODE_VR, V_CTF | V_REF | V_MANY>(ts, a, smem, s, nullptr, nullptr)
+                    : launch_ts<MODE_VR, V_CTF | V_REF>(ts, a, smem, s, nullptr, nullptr);
+    default: return launch_ts<MODE_VR, V_MANY>(ts, a, smem, s, nullptr, nullptr);
     }
 }
 
@@ -449,8 +462,12 @@ int batch_launch_t(const ytgb_batch_entry *d, int n, int total, int *queue, int 
                    cudaStream_t s) {
     // smem > 0: every entry shares the transfer function (ytgb_batch_plan),
     // staged in shared memory; 0: tables read from global memory
-    const bool staged = smem > 0 && (MODE == MODE_VR || MODE == MODE_LIGHT);
-    auto kernel = staged ? batch_kernel<MODE, VAR, TS, true> : batch_kernel<MODE, VAR, TS, false>;
+    constexpr bool tables = MODE == MODE_VR || MODE == MODE_LIGHT;
+    const bool staged = smem > 0 && tables;
+    auto kernel = batch_kernel<MODE, VAR, TS, false>;
+    if constexpr (tables) {
+        if (staged) kernel = batch_kernel<MODE, VAR, TS, true>;
+    }
     if (!staged) smem = 0;
     if (int st = set_smem(kernel, smem)) return st;
     if (blocks <= 0) {
@@ -491,17 +508,19 @@ extern "C" int ytgb_render(const ytgb_render_args *a, void *stream) {
     if (a->kind == YTGB_LIGHT_SOURCE) {
         size_t smem = 0;
         if ((st = tf_check(a->tf, &smem, false))) return st;
-        return (var & V_REF) ? launch_ts<MODE_LIGHT, V_REF>(ts, a, smem, s, nullptr, nullptr)
-                             : launch_ts<MODE_LIGHT, 0>(ts, a, smem, s, nullptr, nullptr);
+        return (var & V_REF) ? launch_ts<MODE_LIGHT, V_REF | V_MANY>(ts, a, smem, s, nullptr, nullptr)
+                             : launch_ts<MODE_LIGHT, V_MANY>(ts, a, smem, s, nullptr, nullptr);
     }
     if (a->kind == YTGB_VOLUME_RENDER) {
         size_t smem = 0;
         if ((st = tf_check(a->tf, &smem, a->tf.ctf_fast != 0))) return st;
-        return launch_var<MODE_VR>(var, ts, a, smem, s);
+        return launch_vr(var, ts, a, smem, s);
     }
     switch (a->kind) {
     case YTGB_PROJECTION: return launch_ts<MODE_PROJ, 0>(ts, a, 0, s, nullptr, nullptr);
-    case YTGB_INTERPOLATED_PROJECTION: return launch_ts<MODE_IPROJ, 0>(ts, a, 0, s, nullptr, nullptr);
+    case YTGB_INTERPOLATED_PROJECTION:
+        return a->n_samples != 1 ? launch_ts<MODE_IPROJ, V_MANY>(ts, a, 0, s, nullptr, nullptr)
+                                 : launch_ts<MODE_IPROJ, 0>(ts, a, 0, s, nullptr, nullptr);
     default: return launch_ts<MODE_MIP, 0>(ts, a, 0, s, nullptr, nullptr);
     }
 }
