@@ -205,6 +205,13 @@ int ytgb_check_error(const int32_t *d_error, void *stream);
 int ytgb_brick_rects(const ytgb_view *view, const ytgb_brick *bricks, int32_t n_bricks,
                      const int32_t *order, int32_t n_order, int32_t *rects);
 
+/* The same on the device (the same integers), for a caller that launches a
+ * render next on this stream: d_bricks, d_order and d_rects (16-byte aligned)
+ * are device arrays.  An order entry that names no brick gets an empty
+ * rectangle. */
+int ytgb_brick_rects_device(const ytgb_view *view, const ytgb_brick *d_bricks, int32_t n_bricks,
+                            const int32_t *d_order, int32_t n_order, int32_t *d_rects, void *stream);
+
 /* ---- host: transfer function --------------------------------------------- */
 /* Replaces FIT_initialize_table (field_interpolation_tables.pxd:44-61) for the
  * tables of VolumeRenderSampler.__cinit__ (image_samplers.pyx:425-447).

@@ -178,6 +178,8 @@ SIGNATURES = {
     "ytgb_check_error": (C.c_int, [C.c_void_p, C.c_void_p]),
     "ytgb_brick_rects": (C.c_int, [C.POINTER(View), C.POINTER(Brick), C.c_int32, C.c_void_p, C.c_int32,
                                    C.c_void_p]),
+    "ytgb_brick_rects_device": (C.c_int, [C.POINTER(View), C.c_void_p, C.c_int32, C.c_void_p, C.c_int32,
+                                          C.c_void_p, C.c_void_p]),
     "ytgb_tf_pack": (C.c_int, [C.c_int32, C.POINTER(_dp), C.POINTER(C.c_int32), _dp, C.POINTER(C.c_int32),
                                C.POINTER(C.c_int32), C.POINTER(C.c_int32), C.POINTER(C.c_int32), C.c_int32,
                                C.POINTER(TF), C.c_void_p]),

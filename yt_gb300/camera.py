@@ -84,6 +84,7 @@ class Camera:
     def sampler_params(self):
         if self.lens_type == "plane-parallel":
             p = self._plane_parallel()
+            p["image"] = np.zeros((*self.resolution, 4), dtype="float64")
         else:
             p = self._perspective()
         p["width"] = self.width.copy()
@@ -91,7 +92,6 @@ class Camera:
         return p
 
     def _plane_parallel(self):
-        nx, ny = self.resolution
         return {
             "vp_pos": np.concatenate([self.inv_mat.ravel("F"), self.back_center.ravel()]),
             "vp_dir": self.box_vectors[2],
@@ -99,7 +99,6 @@ class Camera:
             "bounds": (-self.width[0] / 2.0, self.width[0] / 2.0, -self.width[1] / 2.0, self.width[1] / 2.0),
             "x_vec": self.unit_vectors[0],
             "y_vec": self.unit_vectors[1],
-            "image": np.zeros((nx, ny, 4), dtype="float64"),
             "lens_type": "plane-parallel",
         }
 
@@ -140,10 +139,11 @@ class Camera:
         if self.lens_type == "plane-parallel":
             from .image_samplers import make_view
 
-            p = self.sampler_params()
+            p = self._plane_parallel()
             nx, ny = self.resolution
-            v, _, _ = make_view(p["vp_pos"], p["vp_dir"], p["center"], p["bounds"], nx, ny, p["x_vec"],
-                                p["y_vec"], p["width"], p["lens_type"], p["camera_data"])
+            v, _, _ = make_view(p["vp_pos"], p["vp_dir"], p["center"], p["bounds"], nx, ny, p["x_vec"], p["y_vec"],
+                                self.width, p["lens_type"],
+                                np.vstack((self.position, self.width, self.unit_vectors)))
             return v
         nx, ny = self.resolution
         self.width[1] = self.width[0] * (ny / nx)

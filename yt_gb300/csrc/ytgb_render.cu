@@ -495,6 +495,8 @@ int batch_launch_ts(int ts, const ytgb_batch_entry *d, int n, int total, int *qu
 
 }  // namespace
 
+#include "ytgb_rects.cuh"
+
 extern "C" int ytgb_render(const ytgb_render_args *a, void *stream) {
     int st = check_args(a, false);
     if (st) return st;

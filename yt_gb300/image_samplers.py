@@ -378,12 +378,11 @@ class ImageSampler:
         waits for that once the bricks are gathered.  As with yt's sampler,
         a render that fails (an error word raised below) may have written
         part of the image."""
-        # (the device gather runs while the rectangles are computed: pending
-        # keeps the bricks alive and the stream is synchronised below before
-        # they may change)
+        # (the device gather runs on: pending keeps the bricks alive and the
+        # stream is synchronised below before they may change; the pixel
+        # rectangles are formed on the device behind it)
         bricks = BrickSet(pending, device=dev, with_lo=self._with_lo, direct=True, sync=False)
         order = np.arange(len(pending), dtype=np.int32)
-        rects = bricks.rects(self._view, order)
         t_bricks = time.perf_counter()
         pre = self._await_prefault(img, L)
         t1 = time.perf_counter()
@@ -393,7 +392,7 @@ class ImageSampler:
         keep = []
         _render(bricks, self._view, order, self.kind, img, tf=self._tf(), zbuffer=zb, n_samples=self.n_samples,
                 flags=self.flags, counters=counters, error=error, px_pos=self._px_pos, px_dir=self._px_dir,
-                light=self._light(), keep=keep, rects=rects)
+                light=self._light(), keep=keep)
         t2 = time.perf_counter()
         _lib.check(L.ytgb_check_error(error.data_ptr(), stream.cuda_stream), "render")
         keep.clear()
@@ -410,8 +409,7 @@ class ImageSampler:
             h2d += self._px_pos.nbytes + self._px_dir.nbytes
         self.last_h2d_bytes = int(bricks.upload_bytes + h2d + 20 * len(pending))
         self.last_d2h_bytes = int(img.nbytes + 4 * 8)
-        # pack: bricks gathered and rectangles computed (bricks_at), image
-        # pages faulted in; launch; render: until the image is written;
+        # pack: bricks gathered (bricks_at), image pages faulted in; launch; render: until the image is written;
         # download: the counters
         self.last_timings = {"pack_ms": 1e3 * (t1 - t0), "launch_ms": 1e3 * (t2 - t1), "render_ms": 1e3 * (t3 - t2),
                              "download_ms": 1e3 * (t4 - t3), "bricks_at_ms": 1e3 * (t_bricks - t0)}

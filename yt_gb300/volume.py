@@ -371,6 +371,22 @@ class BrickSet:
                 "ytgb_brick_layout")
         return desc, desc["field_stride"].copy(), desc["data_offset"].copy(), int(total.value), bounds
 
+    def device_table(self, view: _lib.View, order: np.ndarray, stream) -> torch.Tensor:
+        """The table one render reads -- the order's pixel rectangles (4 int32
+        each, ``ytgb_brick_rects_device``), then the order -- formed on the
+        device, in flight on ``stream``."""
+        n = order.size
+        host = _pinned((n,), torch.int32, self.device)
+        host.numpy()[:] = order
+        with torch.cuda.stream(stream):
+            tab = torch.empty(5 * n, dtype=torch.int32, device=self.device)
+            tab[4 * n:].copy_(host, non_blocking=True)
+        base = tab.data_ptr()
+        _lib.check(_lib.lib().ytgb_brick_rects_device(C.byref(view), self.desc.data_ptr(), self.n, base + 16 * n, n,
+                                                      base, C.c_void_p(stream.cuda_stream)),
+                   "ytgb_brick_rects_device")
+        return tab
+
     def rects(self, view: _lib.View, order: np.ndarray) -> np.ndarray:
         """Per-order-entry pixel rectangles (ytgb_brick_rects)."""
         order = np.ascontiguousarray(order, dtype=np.int32)
@@ -431,12 +447,11 @@ def check_inputs(bricks: BrickSet, view: _lib.View, order, kind, image=None, zbu
     dims^3 (image_samplers.pyx:341, :384-385, :465-466)."""
     if order.size and (order.min() < 0 or order.max() >= bricks.n):
         raise ValueError("order entry out of range")
-    used = np.unique(order) if order.size else order
     need = (bricks.verts if kind in (_lib.VOLUME_RENDER, _lib.INTERPOLATED_PROJECTION, _lib.LIGHT_SOURCE)
             else bricks.cells)
-    short = used[bricks.min_elems[used] < need[used]] if used.size else used
+    short = order[bricks.min_elems[order] < need[order]]
     if short.size:
-        k = int(short[0])
+        k = int(short.min())
         raise ValueError(f"brick {k} has {bricks.min_elems[k]} values per field; this sampler reads {need[k]}")
     nx, ny = view.nx, view.ny
     for t in (image, zbuffer):
@@ -511,8 +526,8 @@ def render(bricks: BrickSet, view: _lib.View, order: np.ndarray, kind: int, imag
     device tensor updated in place -- or, on a device that reads and writes
     pageable host memory, a host array (likewise ``zbuffer``); ``tf`` a
     PackedTF for volume rendering; ``tables`` the resident table of
-    :func:`render_tables` for this view and order (else it is built from
-    ``rects`` and uploaded for this launch).
+    :func:`render_tables` for this view and order (else it is formed on the
+    device, or uploaded from ``rects`` where given).
     Device temporaries that must outlive the asynchronous launch are appended
     to ``keep`` when given."""
     dev = bricks.device
@@ -520,9 +535,9 @@ def render(bricks: BrickSet, view: _lib.View, order: np.ndarray, kind: int, imag
     check_inputs(bricks, view, order, kind, image, zbuffer, px_pos, px_dir)
     if stream is None:
         stream = torch.cuda.current_stream(dev)
-    if tables is None:
-        if rects is None:
-            rects = bricks.rects(view, order)
+    if tables is None and rects is None:
+        tab_d = bricks.device_table(view, order, stream)
+    elif tables is None:
         with torch.cuda.stream(stream):
             tab_d = torch.from_numpy(_table(rects, order)).pin_memory().to(dev, non_blocking=True)
     else:
