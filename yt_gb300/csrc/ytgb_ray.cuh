@@ -255,6 +255,49 @@ YTGB_HD void step_advance(AxisStep &s, double d) {
     step_prepare(s, d);
 }
 
+// a / b, correctly rounded, on the integer pipe: about sixty instructions where
+// the float64 division takes ten of the float64 pipe's at 64 cycles each.  The
+// quotient of the 53-bit mantissas from a float32 reciprocal improved by
+// Newton's iteration in fixed point (two terms of the series), then its exact
+// remainder: every product below is needed modulo 2^64 only, since 2^83 and 2^105
+// vanish there and the differences formed are below 2^63.  An exact half does
+// not occur in a quotient of two numbers of one precision.  Zero, subnormal,
+// infinite and NaN operands and results near them take the division itself.
+YTGB_HD double quotient(double a, double b) {
+    const unsigned long long ab = (unsigned long long)dbits(a), bb = (unsigned long long)dbits(b);
+    const int ea = (int)(ab >> 52) & 0x7ff, eb = (int)(bb >> 52) & 0x7ff, e = ea - eb + 1022;
+    if ((unsigned)(ea - 1) > 2044u || (unsigned)(eb - 1) > 2044u || (unsigned)(e - 1) > 2043u) return ddiv(a, b);
+    const unsigned long long A = (ab & (unsigned long long)MANT52) | (1ull << 52),
+                             B = (bb & (unsigned long long)MANT52) | (1ull << 52);
+    // Y / 2^31 = 2^52 / B to 2^-22
+    const float y = frcp(ffrom(0x3f800000u | (unsigned)((B >> 29) & 0x7fffffu)));
+    const unsigned Y = (unsigned)fmul(y, 2147483648.0f);
+    // 2^83 - B Y = D, |D| < 2^62: 2^105 / B = 2^22 Y (1 + D / 2^83 + (D / 2^83)^2 + ...), to a few units
+    const long long D = -(long long)(B * Y);
+    const long long d = D >> 30;
+    const long long z1 = ((long long)Y * d) >> 31, z2 = (z1 * d) >> 53;
+    const unsigned long long Z = ((unsigned long long)Y << 22) + (unsigned long long)(z1 + z2);
+    const int k = A < B ? 53 : 52;  // the quotient A 2^k / B lies in [2^52, 2^53)
+#ifdef __CUDA_ARCH__
+    unsigned long long q = __umul64hi(A << 11, Z << 10) >> (62 - k);
+#else
+    unsigned long long q = (unsigned long long)(((unsigned __int128)(A << 11) * (Z << 10)) >> 64) >> (62 - k);
+#endif
+    long long R = (long long)((A << k) - q * B);
+    const long long Bs = (long long)B;
+    while (R < 0) {
+        R += Bs;
+        q--;
+    }
+    while (R >= Bs) {
+        R -= Bs;
+        q++;
+    }
+    q += 2 * R > Bs ? 1 : 0;
+    return dfrom((long long)(((ab ^ bb) & 0x8000000000000000ull) +
+                             ((unsigned long long)(e + (k == 52 ? 1 : 0) - 1) << 52) + q));
+}
+
 struct Ray {
     double pos[3];
     double dir[3];
@@ -274,20 +317,35 @@ struct Ray {
 static_assert(sizeof(Ray) == 184, "Ray: an odd number of 8-byte words");
 
 // The view's derived per-view constants (host, before a launch): the
-// perspective lens's linspace steps and normal * width[2], the same float64
-// operations make_ray would repeat per pixel.
+// perspective lens's linspace steps and normal * width[2], or the plane-parallel
+// lens's inverse direction in their place (0 for a zero component): the same
+// float64 operations make_ray would repeat per pixel, there at 64 cycles of the
+// float64 pipe each (about nine to a division).
 inline void view_derive(ytgb_view &v) {
     v.lin_step[0] = v.nx > 1 ? 1.0 / (double)(v.nx - 1) : 0.0;
     v.lin_step[1] = v.ny > 1 ? 1.0 / (double)(v.ny - 1) : 0.0;
-    for (int i = 0; i < 3; i++) v.normal_w2[i] = v.vp_pos[9 + i] * v.vp_dir[2];
+    for (int i = 0; i < 3; i++)
+        v.normal_w2[i] = v.lens == YTGB_LENS_PLANE_PARALLEL ? (v.vp_dir[i] != 0.0 ? 1.0 / v.vp_dir[i] : 0.0)
+                                                            : v.vp_pos[9 + i] * v.vp_dir[2];
+}
+
+// (float)x on the integer pipe (the conversion takes the float64 pipe) where x
+// and the result are normal
+YTGB_HD float narrow(double x) {
+    const long long b = dbits(x);
+    const unsigned e = (unsigned)(b >> 52) & 0x7ffu;
+    if (e - 897u > 253u - 1u) return (float)x;
+    const unsigned long long m = (unsigned long long)b & 0x7fffffffffffffffull;
+    const unsigned r = (unsigned)((m + 0x0fffffffull + ((m >> 29) & 1ull)) >> 29);  // to nearest, ties to even
+    return ffrom(((unsigned)(b >> 32) & 0x80000000u) | (r - (896u << 23)));
 }
 
 // generate_vector_info_plane_parallel (lenses.pyx:179-192) and
 // generate_vector_info_null (lenses.pyx:196-207)
 YTGB_HD void make_ray(const ytgb_view &v, int vi, int vj, Ray &r) {
     if (v.lens == YTGB_LENS_PLANE_PARALLEL) {
-        double px = dsub(ddiv(dmul(v.width[0], (double)vi), dsub((double)v.nx, 1.0)), ddiv(v.width[0], 2.0));
-        double py = dsub(ddiv(dmul(v.width[1], (double)vj), dsub((double)v.ny, 1.0)), ddiv(v.width[1], 2.0));
+        double px = dsub(ddiv(dmul(v.width[0], (double)vi), dsub((double)v.nx, 1.0)), dmul(v.width[0], 0.5));
+        double py = dsub(ddiv(dmul(v.width[1], (double)vj), dsub((double)v.ny, 1.0)), dmul(v.width[1], 0.5));
         r.pos[0] = dadd(dadd(dmul(v.vp_pos[0], px), dmul(v.vp_pos[3], py)), v.vp_pos[9]);
         r.pos[1] = dadd(dadd(dmul(v.vp_pos[1], px), dmul(v.vp_pos[4], py)), v.vp_pos[10]);
         r.pos[2] = dadd(dadd(dmul(v.vp_pos[2], px), dmul(v.vp_pos[5], py)), v.vp_pos[11]);
@@ -321,9 +379,10 @@ YTGB_HD void make_ray(const ytgb_view &v, int vi, int vj, Ray &r) {
         if (r.dir[i] < 0) r.step[i] = -1;
         else if (r.dir[i] == 0.0) r.step[i] = 0;
         else r.step[i] = 1;
-        r.iv[i] = r.step[i] != 0 ? ddiv(1.0, r.dir[i]) : 0.0;
-        r.fpos[i] = (float)r.pos[i];
-        r.fdir[i] = (float)r.dir[i];
+        if (v.lens == YTGB_LENS_PLANE_PARALLEL) r.iv[i] = v.normal_w2[i];
+        else r.iv[i] = r.step[i] != 0 ? ddiv(1.0, r.dir[i]) : 0.0;
+        r.fpos[i] = narrow(r.pos[i]);
+        r.fdir[i] = narrow(r.dir[i]);
         r.ifd[i] = frcp(r.fdir[i]);  // = 1.0f / fdir, correctly rounded
         r.td_dds[i] = -1.0;          // no brick has a negative dds
         r.td[i] = 0.0;
@@ -608,9 +667,10 @@ YTGB_HD int walk_setup_face(const BrickF &bf, const ytgb_brick *bp, const double
 // walk_volume set-up: the common walk's form where float32 proves it, else
 // the general one.
 YTGB_HD bool walk_setup(const BrickF &bf, const ytgb_brick *bp, const double *bounds, const Ray &r,
-                        const float ifd[3], double max_t, long long kmax, Walk &w) {
+                        const float ifd[3], double max_t, float max_tf, long long kmax, Walk &w) {
     const int s = walk_setup_face(bf, bp, bounds, r, ifd, kmax, w);
-    if (__builtin_expect(s < 0, 0)) return walk_setup_general(bf, bp, bounds, r, ifd, max_t, kmax, w);
+    if (__builtin_expect(s < 0, 0))
+        return !surely_misses(bf, r, ifd, max_tf) && walk_setup_general(bf, bp, bounds, r, ifd, max_t, kmax, w);
     return s > 0;
 }
 
@@ -1447,12 +1507,23 @@ YTGB_HD void grey_sel2(float &h0, float &l0, float &h1, float &l1, float dt, F2 
     l1 = in ? (small ? f2y(r) : 0.0f) : l1;
 }
 
+// A value's bin, clipped to the table's (a NaN's is 0: it is out of range): the
+// unsigned conversion takes what is below 0, and NaN, to 0.
+YTGB_HD int ctf_index(const ytgb_tf &tf, float val) {
+    const float q = fmul(fsub(val, tf.b0[0]), tf.idbin[0]);
+#ifdef __CUDA_ARCH__
+    const unsigned bin = __float2uint_rz(q);
+#else
+    const unsigned bin = q >= 1.0f ? (q < 4294967040.0f ? (unsigned)q : 0xffffffffu) : 0u;
+#endif
+    const unsigned top = (unsigned)(tf.nbins[0] - 2);
+    return (int)(bin < top ? bin : top);
+}
+
 // The three channels' emission times alpha of a ColorTransferFunction from its
 // tables as ytgb_tf_pack lays them out (in global or shared memory).
 YTGB_HD void ctf_emission(const ytgb_tf &tf, const float4 *tab, float val, float e[3]) {
-    float q = fmul(fsub(val, tf.b0[0]), tf.idbin[0]);
-    q = fminf(fmaxf(q, 0.0f), (float)(tf.nbins[0] - 2));
-    const float4 *t = tab + (int)q;
+    const float4 *t = tab + ctf_index(tf, val);
     const float4 t3 = t[3 * tf.nbins_max];
     const float dd = fsub(fsub(val, t3.z), t3.w);
     const float al = ffma(dd, t3.y, t3.x);
@@ -1472,9 +1543,7 @@ YTGB_HD bool ctf_in(const ytgb_tf &tf, float val) { return val < tf.hi_excl[0] &
 template <bool COMP, bool TG>
 YTGB_HD void shade_ctf(const ytgb_tf &tf, const float4 *s_tab, float val, bool in, bool grey, float dtf,
                        RayState &st) {
-    float q = fmul(fsub(val, tf.b0[0]), tf.idbin[0]);
-    q = fminf(fmaxf(q, 0.0f), (float)(tf.nbins[0] - 2));  // a NaN q gives bin 0 (the sample is then out of range)
-    const int bin = (int)q;
+    const int bin = ctf_index(tf, val);
     float4 Y, D;
     float2 Z;
     ctf_bin<TG>(s_tab, tf.nbins_max, bin, Y, D, Z);
@@ -1806,11 +1875,10 @@ YTGB_HD void walk_brick(const ytgb_render_args &a, const float4 *s_tab, Ray &r, 
     // is within two float32 roundings of the quotient; their margins are 1e-5
     // and 1e-4 of the operands' scale)
     const float ifd[3] = {r.ifd[0], r.ifd[1], r.ifd[2]};
-    if (surely_misses(bf, r, ifd, st.max_tf)) return;
     const double max_t = st.max_t;
     const long long kmax = dkey(st.max_t);
     Walk w;
-    if (!walk_setup(bf, bp, a.bounds, r, ifd, max_t, kmax, w)) return;
+    if (!walk_setup(bf, bp, a.bounds, r, ifd, max_t, st.max_tf, kmax, w)) return;
     st.walks++;
     CellCtx c;
     c.nf = ldg(&bp->n_fields);

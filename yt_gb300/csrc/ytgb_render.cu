@@ -438,6 +438,13 @@ int launch_ts(int ts, const ytgb_render_args *a, size_t smem, cudaStream_t s, un
     }
 }
 
+// The kernels with sample_many render in one tile shape, 16 x 8 (the fastest of
+// every class measured; the image is the same in every shape).
+template <int MODE, int VAR>
+int launch_many(const ytgb_render_args *a, size_t smem, cudaStream_t s) {
+    return launch<MODE, VAR | V_MANY, 1>(a, smem, s, nullptr, nullptr);
+}
+
 int tile_shape_of(uint32_t flags) { return (int)((flags >> YTGB_FLAG_TILE_SHIFT) & 0xfu); }
 
 // Volume rendering: the launch's variant, with sample_many where the
@@ -447,13 +454,13 @@ int launch_vr(int var, int ts, const ytgb_render_args *a, size_t smem, cudaStrea
     const bool many = a->n_samples != 1 || a->masks;
     switch (var) {
     case V_CTF:
-        return many ? launch_ts<MODE_VR, V_CTF | V_MANY>(ts, a, smem, s, nullptr, nullptr)
+        return many ? launch_many<MODE_VR, V_CTF>(a, smem, s)
                     : launch_ts<MODE_VR, V_CTF>(ts, a, smem, s, nullptr, nullptr);
-    case V_REF: return launch_ts<MODE_VR, V_REF | V_MANY>(ts, a, smem, s, nullptr, nullptr);
+    case V_REF: return launch_many<MODE_VR, V_REF>(a, smem, s);
     case V_CTF | V_REF:
-        return many ? launch_ts<MODE_VR, V_CTF | V_REF | V_MANY>(ts, a, smem, s, nullptr, nullptr)
+        return many ? launch_many<MODE_VR, V_CTF | V_REF>(a, smem, s)
                     : launch_ts<MODE_VR, V_CTF | V_REF>(ts, a, smem, s, nullptr, nullptr);
-    default: return launch_ts<MODE_VR, V_MANY>(ts, a, smem, s, nullptr, nullptr);
+    default: return launch_many<MODE_VR, 0>(a, smem, s);
     }
 }
 
@@ -510,8 +517,7 @@ extern "C" int ytgb_render(const ytgb_render_args *a, void *stream) {
     if (a->kind == YTGB_LIGHT_SOURCE) {
         size_t smem = 0;
         if ((st = tf_check(a->tf, &smem, false))) return st;
-        return (var & V_REF) ? launch_ts<MODE_LIGHT, V_REF | V_MANY>(ts, a, smem, s, nullptr, nullptr)
-                             : launch_ts<MODE_LIGHT, V_MANY>(ts, a, smem, s, nullptr, nullptr);
+        return (var & V_REF) ? launch_many<MODE_LIGHT, V_REF>(a, smem, s) : launch_many<MODE_LIGHT, 0>(a, smem, s);
     }
     if (a->kind == YTGB_VOLUME_RENDER) {
         size_t smem = 0;
@@ -521,7 +527,7 @@ extern "C" int ytgb_render(const ytgb_render_args *a, void *stream) {
     switch (a->kind) {
     case YTGB_PROJECTION: return launch_ts<MODE_PROJ, 0>(ts, a, 0, s, nullptr, nullptr);
     case YTGB_INTERPOLATED_PROJECTION:
-        return a->n_samples != 1 ? launch_ts<MODE_IPROJ, V_MANY>(ts, a, 0, s, nullptr, nullptr)
+        return a->n_samples != 1 ? launch_many<MODE_IPROJ, 0>(a, 0, s)
                                  : launch_ts<MODE_IPROJ, 0>(ts, a, 0, s, nullptr, nullptr);
     default: return launch_ts<MODE_MIP, 0>(ts, a, 0, s, nullptr, nullptr);
     }
