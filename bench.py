@@ -28,6 +28,7 @@ Arms:
 from __future__ import annotations
 
 import argparse
+import ctypes
 import json
 import os
 import subprocess
@@ -306,6 +307,9 @@ def run_ours(args):
     r.counters.zero_()
     times = []
     launches = 0
+    need = ctypes.c_int64()
+    _lib.check(_lib.lib().ytgb_render_scratch(ctypes.byref(view), order.size, ctypes.byref(need)), "scratch")
+    per_render = 3 if need.value else 1  # the render; the order of its tiles (their costs, the sort)
     if world > 1:
         torch.distributed.barrier()
     torch.cuda.synchronize()
@@ -322,7 +326,7 @@ def run_ours(args):
                     error=r.error, px_pos=px_pos, px_dir=px_dir, stream=stream, tables=tables, keep=keep,
                     flags=tflags)
             e1.record(stream)
-            launches += 1
+            launches += per_render
             times.append((e0, e1))
         torch.cuda.synchronize()
         t_wall = time.perf_counter() - t_wall0

@@ -229,6 +229,16 @@ int ytgb_tf_pack(int32_t n_fits, const double *const *values, const int32_t *nbi
  * ImageSampler.__call__ -> cast_through_kdtree -> walk_volume -> sample. */
 int ytgb_render(const ytgb_render_args *args, void *stream);
 
+/* The same render with scratch memory of the device (4-byte aligned), in
+ * which the order of the blocks' tiles is formed, on the same stream, so that
+ * the tiles with most work start first; the image is the same.
+ * ytgb_render_scratch (host) writes the bytes to hand over, 0 where no order
+ * is formed (few tiles, one brick, past 65535 tiles); with null or smaller
+ * scratch memory the tiles are taken in grid order, as by ytgb_render.  The
+ * memory must stay the render's until it has run. */
+int ytgb_render_scratch(const ytgb_view *view, int32_t n_order, int64_t *bytes);
+int ytgb_render_scheduled(const ytgb_render_args *args, void *scratch, int64_t bytes, void *stream);
+
 /* Traversal trace: for every pixel, an FNV-1a hash over (brick, index[3],
  * enter_t bits, exit_t bits) of every cell walk_volume (grid_traversal.pyx:
  * 26-140) hands to the sampler, and the visit count.  hashes/counts are
@@ -416,6 +426,12 @@ void ytgb_octree_destroy(void *tree);
  * reference reads per-pixel ray arrays).  args->data must be o->verts;
  * bricks, order and rects are unused. */
 int ytgb_render_octree(const ytgb_render_args *args, const ytgb_octree_args *o, void *stream);
+
+/* The same with scratch memory for the order of the blocks' tiles, as
+ * ytgb_render_scheduled (ytgb_octree_scratch: 0 also for per-pixel rays). */
+int ytgb_octree_scratch(const ytgb_view *view, int32_t n_cells, int64_t *bytes);
+int ytgb_render_octree_scheduled(const ytgb_render_args *args, const ytgb_octree_args *o, void *scratch,
+                                 int64_t bytes, void *stream);
 /* Traversal trace of the octree path: per pixel an FNV-1a hash over (cell
  * key, enter t bits, exit t bits) of every cell sampled, and the count. */
 int ytgb_trace_octree(const ytgb_render_args *args, const ytgb_octree_args *o, unsigned long long *hashes,

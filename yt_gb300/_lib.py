@@ -184,6 +184,8 @@ SIGNATURES = {
                                C.POINTER(C.c_int32), C.POINTER(C.c_int32), C.POINTER(C.c_int32), C.c_int32,
                                C.POINTER(TF), C.c_void_p]),
     "ytgb_render": (C.c_int, [C.POINTER(RenderArgs), C.c_void_p]),
+    "ytgb_render_scratch": (C.c_int, [C.POINTER(View), C.c_int32, C.POINTER(C.c_int64)]),
+    "ytgb_render_scheduled": (C.c_int, [C.POINTER(RenderArgs), C.c_void_p, C.c_int64, C.c_void_p]),
     "ytgb_trace": (C.c_int, [C.POINTER(RenderArgs), C.c_void_p, C.c_void_p, C.c_void_p]),
     "ytgb_batch_plan": (C.c_int, [C.POINTER(BatchEntry), C.c_int32, C.c_int32, C.POINTER(C.c_int32),
                                   C.POINTER(C.c_int32)]),
@@ -202,6 +204,8 @@ SIGNATURES = {
     "ytgb_octree_nodes": (C.c_int, [C.c_void_p, C.c_void_p]),
     "ytgb_octree_destroy": (None, [C.c_void_p]),
     "ytgb_render_octree": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p]),
+    "ytgb_octree_scratch": (C.c_int, [C.POINTER(View), C.c_int32, C.POINTER(C.c_int64)]),
+    "ytgb_render_octree_scheduled": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p]),
     "ytgb_offaxis_cells": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p]),
     "ytgb_offaxis_sums": (C.c_int, [C.c_void_p] + [C.c_int32] * 5 + [C.c_void_p, C.c_void_p]),
     "ytgb_offaxis_cells_sums": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),

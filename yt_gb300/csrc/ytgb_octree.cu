@@ -12,6 +12,7 @@
 #include "ytgb.h"
 #include "ytgb_internal.h"
 #include "ytgb_octree.cuh"
+#include "ytgb_schedule.cuh"
 
 namespace {
 
@@ -37,7 +38,7 @@ static_assert(sizeof(ytgb_onode) == sizeof(ONode), "ytgb_onode layout");
 // 1.85, to 6 1.91.
 template <int MODE, int CTF>
 __global__ void __launch_bounds__(OBLOCK) octree_kernel(const ytgb_render_args a, const ytgb_octree_args oa,
-                                                         unsigned long long *hashes, long long *counts) {
+                                                         const unsigned short *tiles, unsigned long long *hashes, long long *counts) {
     extern __shared__ float4 s_tab[];
     __shared__ unsigned long long s_cnt[4];
     const int tid = threadIdx.x;
@@ -62,8 +63,10 @@ __global__ void __launch_bounds__(OBLOCK) octree_kernel(const ytgb_render_args a
     const ytgb_view &v = a.view;
     const int tiles_y = (v.ny + OTILE_Y - 1) / OTILE_Y;
     const int warp = tid >> 5, lane = tid & 31;
-    const int vi = (int)(blockIdx.x / tiles_y) * OTILE_X + (warp & 1) * 8 + (lane & 7);
-    const int vj = (int)(blockIdx.x % tiles_y) * OTILE_Y + (warp >> 1) * 4 + (lane >> 3);
+    // tiles: the tile of each block, the heavy ones first; null for grid order
+    const unsigned tile = tiles ? __ldg(tiles + blockIdx.x) : blockIdx.x;
+    const int vi = (int)(tile / tiles_y) * OTILE_X + (warp & 1) * 8 + (lane & 7);
+    const int vj = (int)(tile % tiles_y) * OTILE_Y + (warp >> 1) * 4 + (lane >> 3);
     const bool active = vi < v.nx && vj < v.ny;
     const long long p = (long long)vi * v.ny + vj;
     RayState st;
@@ -105,6 +108,57 @@ __global__ void __launch_bounds__(OBLOCK) octree_kernel(const ytgb_render_args a
         __syncthreads();
         if (tid < 4 && s_cnt[tid]) atomicAdd(a.counters + tid, s_cnt[tid]);
     }
+}
+
+// cost[tile] += the share of the tile that each cell covers on the image of a
+// perspective camera, in sixty-fourths: the cells a ray of the tile crosses.
+// In float32, from the cell's centre and half its widest side: an estimate
+// that decides nothing but the tiles' order.  One thread per cell; a cell
+// beside or behind the camera, or over more than 256 tiles, is left out.
+constexpr int COST_BLOCK = 256;
+
+__global__ void __launch_bounds__(COST_BLOCK)
+cell_cost_kernel(const ytgb_view v, const double *edges, int n_cells, int tiles_x, int tiles_y, unsigned *cost) {
+    const int k = blockIdx.x * COST_BLOCK + threadIdx.x;
+    if (k >= n_cells) return;
+    float d[3], half = 0.f;
+    for (int i = 0; i < 3; i++) {
+        const float le = (float)(edges[9ll * k + i] - v.vp_pos[i]), re = (float)(edges[9ll * k + 3 + i] - v.vp_pos[i]);
+        d[i] = 0.5f * (le + re);
+        half = fmaxf(half, 0.5f * (re - le));
+    }
+    float p[3];
+    for (int j = 0; j < 3; j++)
+        p[j] = d[0] * (float)v.vp_pos[3 + 3 * j] + d[1] * (float)v.vp_pos[4 + 3 * j] + d[2] * (float)v.vp_pos[5 + 3 * j];
+    if (!(p[2] > 2.f * half)) return;
+    // pixels per unit across the image at the cell's depth
+    const float sx = (float)v.nx * (float)v.vp_dir[2] / ((float)v.vp_dir[0] * p[2]);
+    const float sy = (float)v.ny * (float)v.vp_dir[2] / ((float)v.vp_dir[1] * p[2]);
+    const float hx = half * sx / OTILE_X, hy = half * sy / OTILE_Y;  // in tiles
+    const float cx = (p[0] * sx + 0.5f * v.nx) / OTILE_X, cy = (p[1] * sy + 0.5f * v.ny) / OTILE_Y;
+    const int x0 = (int)fminf(fmaxf(cx - hx, 0.f), (float)tiles_x), x1 = (int)fminf(fmaxf(cx + hx + 1.f, 0.f), (float)tiles_x);
+    const int y0 = (int)fminf(fmaxf(cy - hy, 0.f), (float)tiles_y), y1 = (int)fminf(fmaxf(cy + hy + 1.f, 0.f), (float)tiles_y);
+    const int h = y1 - y0, n = (x1 - x0) * h;
+    if (x1 <= x0 || h <= 0 || n > 256) return;
+    const unsigned w = 1u + (unsigned)(63.f * fminf(2.f * hx / (x1 - x0), 1.f) * fminf(2.f * hy / h, 1.f));
+    for (int i = 0; i < n; i++) atomicAdd(cost + (x0 + i / h) * tiles_y + y0 + i % h, w);
+}
+
+// The order of a launch's tiles (sort_tiles), or null for grid order: without
+// scratch memory, with rays from arrays (no camera to project by), where all
+// blocks are resident at once (4 per SM) and past MAX_SCHEDULED tiles.
+int schedule_cells(const ytgb_render_args &a, const ytgb_octree_args &o, const Scratch &w, cudaStream_t s,
+                   const unsigned short **tiles) {
+    *tiles = nullptr;
+    const int tx = (a.view.nx + OTILE_X - 1) / OTILE_X, ty = (a.view.ny + OTILE_Y - 1) / OTILE_Y;
+    const long long n = (long long)tx * ty;
+    if (!w.mem || w.bytes < scratch_bytes(n) || a.view.lens != YTGB_LENS_PERSPECTIVE || o.n_cells < 2 ||
+        n > MAX_SCHEDULED || n <= 4ll * sm_count())
+        return YTGB_OK;
+    cudaMemsetAsync(w.mem, 0, (size_t)n * sizeof(unsigned), s);
+    cell_cost_kernel<<<(unsigned)((o.n_cells + (long long)COST_BLOCK - 1) / COST_BLOCK), COST_BLOCK, 0, s>>>(
+        a.view, o.edges, o.n_cells, tx, ty, (unsigned *)w.mem);
+    return sort_tiles(w, (int)n, s, tiles, "octree launch");
 }
 
 int octree_checks(const ytgb_render_args *a, const ytgb_octree_args *o, bool trace, size_t *smem) {
@@ -167,8 +221,8 @@ int octree_checks(const ytgb_render_args *a, const ytgb_octree_args *o, bool tra
 }
 
 template <int MODE, int CTF>
-int octree_launch(const ytgb_render_args *a, const ytgb_octree_args *o, size_t smem, cudaStream_t s,
-                  unsigned long long *h, long long *c) {
+int octree_launch(const ytgb_render_args *a, const ytgb_octree_args *o, size_t smem, const Scratch &w,
+                  cudaStream_t s, unsigned long long *h, long long *c) {
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(octree_kernel<MODE, CTF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
@@ -184,7 +238,9 @@ int octree_launch(const ytgb_render_args *a, const ytgb_octree_args *o, size_t s
     }
     ytgb_render_args b = *a;
     view_derive(b.view);
-    octree_kernel<MODE, CTF><<<(unsigned)blocks, OBLOCK, smem, s>>>(b, *o, h, c);
+    const unsigned short *tiles = nullptr;
+    if (int st = schedule_cells(*a, *o, w, s, &tiles)) return st;
+    octree_kernel<MODE, CTF><<<(unsigned)blocks, OBLOCK, smem, s>>>(b, *o, tiles, h, c);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         ytgb_set_error(std::string("octree launch: ") + cudaGetErrorString(e));
@@ -195,19 +251,45 @@ int octree_launch(const ytgb_render_args *a, const ytgb_octree_args *o, size_t s
 
 }  // namespace
 
-extern "C" int ytgb_render_octree(const ytgb_render_args *a, const ytgb_octree_args *o, void *stream) {
+static int octree_with(const ytgb_render_args *a, const ytgb_octree_args *o, const Scratch &w, void *stream) {
     size_t smem = 0;
     if (int st = octree_checks(a, o, false, &smem)) return st;
     cudaStream_t s = (cudaStream_t)stream;
     switch (a->kind) {
     case YTGB_VOLUME_RENDER:
-        return a->tf.ctf_fast ? octree_launch<MODE_VR, 1>(a, o, smem, s, nullptr, nullptr)
-                              : octree_launch<MODE_VR, 0>(a, o, smem, s, nullptr, nullptr);
-    case YTGB_LIGHT_SOURCE: return octree_launch<MODE_LIGHT, 0>(a, o, smem, s, nullptr, nullptr);
-    case YTGB_PROJECTION: return octree_launch<MODE_PROJ, 0>(a, o, 0, s, nullptr, nullptr);
-    case YTGB_INTERPOLATED_PROJECTION: return octree_launch<MODE_IPROJ, 0>(a, o, 0, s, nullptr, nullptr);
-    default: return octree_launch<MODE_MIP, 0>(a, o, 0, s, nullptr, nullptr);
+        return a->tf.ctf_fast ? octree_launch<MODE_VR, 1>(a, o, smem, w, s, nullptr, nullptr)
+                              : octree_launch<MODE_VR, 0>(a, o, smem, w, s, nullptr, nullptr);
+    case YTGB_LIGHT_SOURCE: return octree_launch<MODE_LIGHT, 0>(a, o, smem, w, s, nullptr, nullptr);
+    case YTGB_PROJECTION: return octree_launch<MODE_PROJ, 0>(a, o, 0, w, s, nullptr, nullptr);
+    case YTGB_INTERPOLATED_PROJECTION: return octree_launch<MODE_IPROJ, 0>(a, o, 0, w, s, nullptr, nullptr);
+    default: return octree_launch<MODE_MIP, 0>(a, o, 0, w, s, nullptr, nullptr);
     }
+}
+
+extern "C" int ytgb_render_octree(const ytgb_render_args *a, const ytgb_octree_args *o, void *stream) {
+    return octree_with(a, o, Scratch{nullptr, 0}, stream);
+}
+
+extern "C" int ytgb_octree_scratch(const ytgb_view *view, int32_t n_cells, int64_t *bytes) {
+    if (!view || !bytes || view->nx <= 0 || view->ny <= 0) {
+        ytgb_set_error("ytgb_octree_scratch: null argument or empty image");
+        return YTGB_ERR_INVALID;
+    }
+    const long long n =
+        (((long long)view->nx + OTILE_X - 1) / OTILE_X) * (((long long)view->ny + OTILE_Y - 1) / OTILE_Y);
+    *bytes = n_cells < 2 || view->lens != YTGB_LENS_PERSPECTIVE || n > MAX_SCHEDULED || n <= 4ll * sm_count()
+                 ? 0
+                 : (int64_t)scratch_bytes(n);
+    return YTGB_OK;
+}
+
+extern "C" int ytgb_render_octree_scheduled(const ytgb_render_args *a, const ytgb_octree_args *o, void *scratch,
+                                            int64_t bytes, void *stream) {
+    if (((uintptr_t)scratch & 3) || bytes < 0) {
+        ytgb_set_error("ytgb_render_octree_scheduled: misaligned scratch memory or negative size");
+        return YTGB_ERR_INVALID;
+    }
+    return octree_with(a, o, Scratch{scratch, (size_t)bytes}, stream);
 }
 
 extern "C" int ytgb_trace_octree(const ytgb_render_args *a, const ytgb_octree_args *o, unsigned long long *hashes,
@@ -218,5 +300,5 @@ extern "C" int ytgb_trace_octree(const ytgb_render_args *a, const ytgb_octree_ar
         ytgb_set_error("ytgb_trace_octree: null or misaligned hash / count arrays");
         return YTGB_ERR_INVALID;
     }
-    return octree_launch<MODE_TRACE, 0>(a, o, 0, (cudaStream_t)stream, hashes, counts);
+    return octree_launch<MODE_TRACE, 0>(a, o, 0, Scratch{nullptr, 0}, (cudaStream_t)stream, hashes, counts);
 }

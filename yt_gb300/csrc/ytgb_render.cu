@@ -55,6 +55,7 @@
 #include "ytgb.h"
 #include "ytgb_internal.h"
 #include "ytgb_ray.cuh"
+#include "ytgb_schedule.cuh"
 
 namespace {
 
@@ -226,10 +227,11 @@ __device__ __forceinline__ void warp_tile(const ytgb_render_args &a, int bx, int
     }
 }
 
-// One view, one tile per block (four warps of 32 pixels).
+// One view, one tile per block (four warps of 32 pixels).  tiles: the tile of
+// each block (schedule_tiles), null for grid order.
 template <int MODE, int VAR, int TS>
 __global__ void __launch_bounds__(BLOCK, min_blocks(MODE, VAR))
-render_kernel(const ytgb_render_args a, unsigned long long *hashes, long long *counts) {
+render_kernel(const ytgb_render_args a, const unsigned short *tiles, unsigned long long *hashes, long long *counts) {
     extern __shared__ float4 s_tab[];
     __shared__ TileSmem sm;
     if (MODE == MODE_VR || MODE == MODE_LIGHT) {
@@ -237,7 +239,13 @@ render_kernel(const ytgb_render_args a, unsigned long long *hashes, long long *c
         __syncthreads();
     }
     const int w = threadIdx.x >> 5;
-    warp_tile<MODE, VAR, TS, false>(a, blockIdx.y, blockIdx.x, w, s_tab, sm, threadIdx.x, w, hashes, counts);
+    int bx = blockIdx.y, by = blockIdx.x;
+    if (MODE != MODE_TRACE && tiles) {
+        const unsigned t = __ldg(tiles + (size_t)blockIdx.y * gridDim.x + blockIdx.x);
+        bx = (int)(t / gridDim.x);
+        by = (int)(t % gridDim.x);
+    }
+    warp_tile<MODE, VAR, TS, false>(a, bx, by, w, s_tab, sm, threadIdx.x, w, hashes, counts);
 }
 
 // Many views in one persistent launch: every warp pulls work items -- one
@@ -392,6 +400,58 @@ int tf_check(const ytgb_tf &t, size_t *smem, bool ctf_layout) {
     return YTGB_OK;
 }
 
+// Cost additions a view may take: past it (thousands of bricks that each cover
+// much of the image, as from a camera among them) the widest bricks, which add
+// nearly the same to every tile, are left out.
+constexpr int MAX_COST_ADDS = 1 << 22;
+
+constexpr int COST_BLOCK = 128;
+
+// A walk's set-up counts as twenty cells (with eight the light-source frame took
+// 537 us, with twenty 530; the others the same); a ray crosses about one brick
+// edge of cells.
+__device__ __forceinline__ unsigned walk_cost(const ytgb_brick &b, int n_samples) {
+    long long edge = ((long long)b.dims[0] + b.dims[1] + b.dims[2]) / 3;
+    edge = edge < 1 ? 1 : (edge > 1024 ? 1024 : edge);
+    return 20u + (unsigned)edge * (unsigned)(n_samples > 64 ? 64 : n_samples);
+}
+
+// cost[tile] += the walk cost of every brick whose rectangle meets the tile
+// (one block per ordered brick; tiles numbered along y first)
+__global__ void __launch_bounds__(COST_BLOCK)
+tile_cost_kernel(const int4 *rects, const int32_t *order, const ytgb_brick *bricks, int nx, int ny, int tx, int ty,
+                 int max_tiles, int n_samples, unsigned *cost) {
+    const int k = blockIdx.x;
+    const int4 rc = rects[k];
+    const int tiles_y = (ny + ty - 1) / ty;
+    const int x0 = max(rc.x, 0) / tx, x1 = (min(rc.y, nx) + tx - 1) / tx;
+    const int y0 = max(rc.z, 0) / ty, y1 = (min(rc.w, ny) + ty - 1) / ty;
+    if (rc.x >= rc.y || rc.z >= rc.w || x1 <= x0 || y1 <= y0) return;
+    const int h = y1 - y0, n = (x1 - x0) * h;
+    if (n > max_tiles) return;
+    const unsigned w = walk_cost(bricks[order[k]], n_samples);
+    for (int i = threadIdx.x; i < n; i += COST_BLOCK) atomicAdd(cost + (x0 + i / h) * tiles_y + y0 + i % h, w);
+}
+
+// The order of a launch's tiles in scratch memory, formed on its stream, or
+// null for grid order: without scratch memory for it, with one brick (its
+// tiles differ little), where all blocks are resident at once, and past
+// MAX_SCHEDULED tiles (the last blocks' time weighs little then).
+int schedule_tiles(const ytgb_render_args &a, int tx, int ty, int blocks_per_sm, const Scratch &w, cudaStream_t s,
+                   const unsigned short **tiles) {
+    *tiles = nullptr;
+    const long long n = (long long)((a.view.nx + tx - 1) / tx) * ((a.view.ny + ty - 1) / ty);
+    if (!w.mem || w.bytes < scratch_bytes(n) || a.n_order < 2 || n > MAX_SCHEDULED ||
+        n <= (long long)blocks_per_sm * sm_count())
+        return YTGB_OK;
+    unsigned *cost = (unsigned *)w.mem;
+    cudaMemsetAsync(cost, 0, (size_t)n * sizeof(unsigned), s);
+    tile_cost_kernel<<<(unsigned)a.n_order, COST_BLOCK, 0, s>>>(
+        (const int4 *)a.rects, a.order, a.bricks, a.view.nx, a.view.ny, tx, ty, MAX_COST_ADDS / a.n_order,
+        a.kind == YTGB_PROJECTION || a.kind == YTGB_MIP ? 1 : a.n_samples, cost);
+    return sort_tiles(w, (int)n, s, tiles, "render launch");
+}
+
 template <typename K>
 int set_smem(K kernel, size_t smem) {
     // (static and dynamic shared memory together need the opt-in past 48 KB)
@@ -415,7 +475,8 @@ int launch_status(const char *what) {
 }
 
 template <int MODE, int VAR, int TS>
-int launch(const ytgb_render_args *a, size_t smem, cudaStream_t s, unsigned long long *h, long long *c) {
+int launch(const ytgb_render_args *a, size_t smem, const Scratch &w, cudaStream_t s, unsigned long long *h,
+           long long *c) {
     constexpr int TX = TileShape<TS>::X, TY = TileShape<TS>::Y;
     dim3 grid((a->view.ny + TY - 1) / TY, (a->view.nx + TX - 1) / TX);
     if (grid.y > 65535) {
@@ -425,24 +486,26 @@ int launch(const ytgb_render_args *a, size_t smem, cudaStream_t s, unsigned long
     if (int st = set_smem(render_kernel<MODE, VAR, TS>, smem)) return st;
     ytgb_render_args b = *a;
     view_derive(b.view);
-    render_kernel<MODE, VAR, TS><<<grid, BLOCK, smem, s>>>(b, h, c);
+    const unsigned short *tiles = nullptr;
+    if (int st = schedule_tiles(*a, TX, TY, min_blocks(MODE, VAR), w, s, &tiles)) return st;
+    render_kernel<MODE, VAR, TS><<<grid, BLOCK, smem, s>>>(b, tiles, h, c);
     return launch_status("render launch");
 }
 
 template <int MODE, int VAR>
-int launch_ts(int ts, const ytgb_render_args *a, size_t smem, cudaStream_t s, unsigned long long *h, long long *c) {
+int launch_ts(int ts, const ytgb_render_args *a, size_t smem, const Scratch &w, cudaStream_t s) {
     switch (ts) {
-    case 1: return launch<MODE, VAR, 1>(a, smem, s, h, c);
-    case 2: return launch<MODE, VAR, 2>(a, smem, s, h, c);
-    default: return launch<MODE, VAR, 0>(a, smem, s, h, c);
+    case 1: return launch<MODE, VAR, 1>(a, smem, w, s, nullptr, nullptr);
+    case 2: return launch<MODE, VAR, 2>(a, smem, w, s, nullptr, nullptr);
+    default: return launch<MODE, VAR, 0>(a, smem, w, s, nullptr, nullptr);
     }
 }
 
 // The kernels with sample_many render in one tile shape, 16 x 8 (the fastest of
 // every class measured; the image is the same in every shape).
 template <int MODE, int VAR>
-int launch_many(const ytgb_render_args *a, size_t smem, cudaStream_t s) {
-    return launch<MODE, VAR | V_MANY, 1>(a, smem, s, nullptr, nullptr);
+int launch_many(const ytgb_render_args *a, size_t smem, const Scratch &w, cudaStream_t s) {
+    return launch<MODE, VAR | V_MANY, 1>(a, smem, w, s, nullptr, nullptr);
 }
 
 int tile_shape_of(uint32_t flags) { return (int)((flags >> YTGB_FLAG_TILE_SHIFT) & 0xfu); }
@@ -450,17 +513,17 @@ int tile_shape_of(uint32_t flags) { return (int)((flags >> YTGB_FLAG_TILE_SHIFT)
 // Volume rendering: the launch's variant, with sample_many where the
 // ColorTransferFunction walks are not all of one sample per unmasked cell
 // (other table sets have no simpler form).
-int launch_vr(int var, int ts, const ytgb_render_args *a, size_t smem, cudaStream_t s) {
+int launch_vr(int var, int ts, const ytgb_render_args *a, size_t smem, const Scratch &w, cudaStream_t s) {
     const bool many = a->n_samples != 1 || a->masks;
     switch (var) {
     case V_CTF:
-        return many ? launch_many<MODE_VR, V_CTF>(a, smem, s)
-                    : launch_ts<MODE_VR, V_CTF>(ts, a, smem, s, nullptr, nullptr);
-    case V_REF: return launch_many<MODE_VR, V_REF>(a, smem, s);
+        return many ? launch_many<MODE_VR, V_CTF>(a, smem, w, s)
+                    : launch_ts<MODE_VR, V_CTF>(ts, a, smem, w, s);
+    case V_REF: return launch_many<MODE_VR, V_REF>(a, smem, w, s);
     case V_CTF | V_REF:
-        return many ? launch_many<MODE_VR, V_CTF | V_REF>(a, smem, s)
-                    : launch_ts<MODE_VR, V_CTF | V_REF>(ts, a, smem, s, nullptr, nullptr);
-    default: return launch_many<MODE_VR, 0>(a, smem, s);
+        return many ? launch_many<MODE_VR, V_CTF | V_REF>(a, smem, w, s)
+                    : launch_ts<MODE_VR, V_CTF | V_REF>(ts, a, smem, w, s);
+    default: return launch_many<MODE_VR, 0>(a, smem, w, s);
     }
 }
 
@@ -504,7 +567,7 @@ int batch_launch_ts(int ts, const ytgb_batch_entry *d, int n, int total, int *qu
 
 #include "ytgb_rects.cuh"
 
-extern "C" int ytgb_render(const ytgb_render_args *a, void *stream) {
+static int render_with(const ytgb_render_args *a, const Scratch &w, void *stream) {
     int st = check_args(a, false);
     if (st) return st;
     cudaStream_t s = (cudaStream_t)stream;
@@ -517,20 +580,49 @@ extern "C" int ytgb_render(const ytgb_render_args *a, void *stream) {
     if (a->kind == YTGB_LIGHT_SOURCE) {
         size_t smem = 0;
         if ((st = tf_check(a->tf, &smem, false))) return st;
-        return (var & V_REF) ? launch_many<MODE_LIGHT, V_REF>(a, smem, s) : launch_many<MODE_LIGHT, 0>(a, smem, s);
+        return (var & V_REF) ? launch_many<MODE_LIGHT, V_REF>(a, smem, w, s) : launch_many<MODE_LIGHT, 0>(a, smem, w, s);
     }
     if (a->kind == YTGB_VOLUME_RENDER) {
         size_t smem = 0;
         if ((st = tf_check(a->tf, &smem, a->tf.ctf_fast != 0))) return st;
-        return launch_vr(var, ts, a, smem, s);
+        return launch_vr(var, ts, a, smem, w, s);
     }
     switch (a->kind) {
-    case YTGB_PROJECTION: return launch_ts<MODE_PROJ, 0>(ts, a, 0, s, nullptr, nullptr);
+    case YTGB_PROJECTION: return launch_ts<MODE_PROJ, 0>(ts, a, 0, w, s);
     case YTGB_INTERPOLATED_PROJECTION:
-        return a->n_samples != 1 ? launch_many<MODE_IPROJ, 0>(a, 0, s)
-                                 : launch_ts<MODE_IPROJ, 0>(ts, a, 0, s, nullptr, nullptr);
-    default: return launch_ts<MODE_MIP, 0>(ts, a, 0, s, nullptr, nullptr);
+        return a->n_samples != 1 ? launch_many<MODE_IPROJ, 0>(a, 0, w, s)
+                                 : launch_ts<MODE_IPROJ, 0>(ts, a, 0, w, s);
+    default: return launch_ts<MODE_MIP, 0>(ts, a, 0, w, s);
     }
+}
+
+extern "C" int ytgb_render(const ytgb_render_args *a, void *stream) {
+    return render_with(a, Scratch{nullptr, 0}, stream);
+}
+
+extern "C" int ytgb_render_scratch(const ytgb_view *view, int32_t n_order, int64_t *bytes) {
+    if (!view || !bytes || view->nx <= 0 || view->ny <= 0) {
+        ytgb_set_error("ytgb_render_scratch: null argument or empty image");
+        return YTGB_ERR_INVALID;
+    }
+    // (of the three tile shapes the one with the most tiles; a launch whose
+    // own shape needs no order takes grid order)
+    long long n = 0;
+    for (int tx : {TileShape<0>::X, TileShape<1>::X, TileShape<2>::X}) {
+        const int ty = BLOCK / tx;
+        const long long k = ((long long)view->nx + tx - 1) / tx * (((long long)view->ny + ty - 1) / ty);
+        if (k <= MAX_SCHEDULED && k > n) n = k;
+    }
+    *bytes = n_order < 2 || n <= 4 * sm_count() ? 0 : (int64_t)scratch_bytes(n);
+    return YTGB_OK;
+}
+
+extern "C" int ytgb_render_scheduled(const ytgb_render_args *a, void *scratch, int64_t bytes, void *stream) {
+    if (((uintptr_t)scratch & 3) || bytes < 0) {
+        ytgb_set_error("ytgb_render_scheduled: misaligned scratch memory or negative size");
+        return YTGB_ERR_INVALID;
+    }
+    return render_with(a, Scratch{scratch, (size_t)bytes}, stream);
 }
 
 extern "C" int ytgb_trace(const ytgb_render_args *a, unsigned long long *hashes, long long *counts, void *stream) {
@@ -540,7 +632,7 @@ extern "C" int ytgb_trace(const ytgb_render_args *a, unsigned long long *hashes,
         ytgb_set_error("ytgb_trace: null hash / count arrays");
         return YTGB_ERR_INVALID;
     }
-    return launch<MODE_TRACE, 0, 0>(a, 0, (cudaStream_t)stream, hashes, counts);
+    return launch<MODE_TRACE, 0, 0>(a, 0, Scratch{nullptr, 0}, (cudaStream_t)stream, hashes, counts);
 }
 
 extern "C" int ytgb_batch_plan(ytgb_batch_entry *entries, int32_t n, int32_t tile_shape, int32_t *total_tiles,

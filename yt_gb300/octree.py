@@ -152,8 +152,15 @@ def render_octree(vol: OctreeVolume, view: _lib.View, kind: int, image: torch.Te
             a.light_rgba[i] = float(rgba[i])
     o = vol.args()
     s = stream or torch.cuda.current_stream(vol.device)
-    _lib.check(_lib.lib().ytgb_render_octree(C.byref(a), C.byref(o), C.c_void_p(s.cuda_stream)),
-               "ytgb_render_octree")
+    L = _lib.lib()
+    need = C.c_int64()
+    _lib.check(L.ytgb_octree_scratch(C.byref(view), vol.n_cells, C.byref(need)), "ytgb_octree_scratch")
+    mem = None
+    if need.value:
+        with torch.cuda.stream(s):  # (its memory goes back to this stream's later work alone)
+            mem = torch.empty(need.value, dtype=torch.uint8, device=vol.device)
+    _lib.check(L.ytgb_render_octree_scheduled(C.byref(a), C.byref(o), _ptr(mem), need.value,
+                                              C.c_void_p(s.cuda_stream)), "ytgb_render_octree")
     return a, o
 
 

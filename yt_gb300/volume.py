@@ -371,16 +371,16 @@ class BrickSet:
                 "ytgb_brick_layout")
         return desc, desc["field_stride"].copy(), desc["data_offset"].copy(), int(total.value), bounds
 
-    def device_table(self, view: _lib.View, order: np.ndarray, stream) -> torch.Tensor:
+    def device_table(self, view: _lib.View, order: np.ndarray, stream, scratch: int = 0) -> torch.Tensor:
         """The table one render reads -- the order's pixel rectangles (4 int32
         each, ``ytgb_brick_rects_device``), then the order -- formed on the
-        device, in flight on ``stream``."""
+        device, in flight on ``stream``; ``scratch`` more bytes follow it."""
         n = order.size
         host = _pinned((n,), torch.int32, self.device)
         host.numpy()[:] = order
         with torch.cuda.stream(stream):
-            tab = torch.empty(5 * n, dtype=torch.int32, device=self.device)
-            tab[4 * n:].copy_(host, non_blocking=True)
+            tab = torch.empty(5 * n + -(-scratch // 4), dtype=torch.int32, device=self.device)
+            tab[4 * n:5 * n].copy_(host, non_blocking=True)
         base = tab.data_ptr()
         _lib.check(_lib.lib().ytgb_brick_rects_device(C.byref(view), self.desc.data_ptr(), self.n, base + 16 * n, n,
                                                       base, C.c_void_p(stream.cuda_stream)),
@@ -535,8 +535,17 @@ def render(bricks: BrickSet, view: _lib.View, order: np.ndarray, kind: int, imag
     check_inputs(bricks, view, order, kind, image, zbuffer, px_pos, px_dir)
     if stream is None:
         stream = torch.cuda.current_stream(dev)
+    L = _lib.lib()
+    need = C.c_int64()
+    # (an image in host memory keeps grid order: its writes cross the link to the CPU)
+    if not isinstance(image, np.ndarray):
+        _lib.check(L.ytgb_render_scratch(C.byref(view), order.size, C.byref(need)), "ytgb_render_scratch")
+    scratch = None
+    if need.value and (tables is not None or rects is not None):
+        with torch.cuda.stream(stream):  # (its memory goes back to this stream's later work alone)
+            scratch = torch.empty(need.value, dtype=torch.uint8, device=dev)
     if tables is None and rects is None:
-        tab_d = bricks.device_table(view, order, stream)
+        tab_d = bricks.device_table(view, order, stream, need.value)
     elif tables is None:
         with torch.cuda.stream(stream):
             tab_d = torch.from_numpy(_table(rects, order)).pin_memory().to(dev, non_blocking=True)
@@ -575,8 +584,9 @@ def render(bricks: BrickSet, view: _lib.View, order: np.ndarray, kind: int, imag
         set_range(args, bricks)
     args.counters = _ptr(counters)
     args.error = _ptr(error)
-    st = _lib.lib().ytgb_render(C.byref(args), C.c_void_p(stream.cuda_stream))
-    _lib.check(st, "ytgb_render")
+    mem = scratch.data_ptr() if scratch is not None else tab_d.data_ptr() + 20 * order.size
+    _lib.check(L.ytgb_render_scheduled(C.byref(args), mem if need.value else None, need.value,
+                                       C.c_void_p(stream.cuda_stream)), "ytgb_render")
     if keep is not None:
         keep.append(tab_d)
     elif tables is None:
