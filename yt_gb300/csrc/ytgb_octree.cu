@@ -34,8 +34,9 @@ static_assert(sizeof(ytgb_onode) == sizeof(ONode), "ytgb_onode layout");
 // sampling together, a 32-byte stack and positive t compared as bits; 2.13
 // with midpoints, float32 pairs and dt on the integer pipe and each cell's
 // entry taken from the last one's exit; 1.82 with parents restored in the
-// iteration that goes on with them.  4 blocks per SM by registers; held to 5
-// 1.85, to 6 1.91.
+// iteration that goes on with them; 1.63 with the heavy tiles first
+// (ytgb_schedule.cuh).  4 blocks per SM by registers; held to 5 1.85 against
+// 1.82, to 6 1.91.
 template <int MODE, int CTF>
 __global__ void __launch_bounds__(OBLOCK) octree_kernel(const ytgb_render_args a, const ytgb_octree_args oa,
                                                          const unsigned short *tiles, unsigned long long *hashes, long long *counts) {
