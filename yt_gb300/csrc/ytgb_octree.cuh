@@ -321,9 +321,11 @@ YTGB_HD bool octree_ray(const ytgb_render_args &a, const OctreeView &o, const fl
         split_pair(r.dir[i], dh[i], dl[i]);
     }
     // the previous cell's exit t and what was formed from it: the next cell's
-    // entry, where the ray goes from cell to cell
-    double t_last = -1.0, x_last = 0.0;
-    float xh_last = 0.0f, xl_last = 0.0f;
+    // entry, where the ray goes from cell to cell.  Before the first cell: of
+    // t = 0 (every t is a possible entry, so what stands here must be its own)
+    double t_last = 0.0, x_last = dmul(0.0, ilen);
+    float xh_last, xl_last;
+    split_pair(x_last, xh_last, xl_last);
     return octree_cast(o, r.pos, r.dir, len, [&](int key, double t_in, double t_out) {
         if (key < 0 || key >= o.n_cells) {
             st.guarded++;
