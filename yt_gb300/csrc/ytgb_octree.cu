@@ -23,6 +23,7 @@ constexpr int OBLOCK = 128;
 // that traverse the octree together stay close on the image, so a warp's
 // lanes follow more of the same path than along a 32-pixel row.
 constexpr int OTILE_X = 16, OTILE_Y = 8;
+constexpr int OCT_COUNTERS = 4;
 
 static_assert(sizeof(ytgb_onode) == sizeof(ONode), "ytgb_onode layout");
 
@@ -41,9 +42,9 @@ template <int MODE, int CTF>
 __global__ void __launch_bounds__(OBLOCK) octree_kernel(const ytgb_render_args a, const ytgb_octree_args oa,
                                                          const unsigned short *tiles, unsigned long long *hashes, long long *counts) {
     extern __shared__ float4 s_tab[];
-    __shared__ unsigned long long s_cnt[4];
+    __shared__ unsigned long long s_cnt[OCT_COUNTERS];
     const int tid = threadIdx.x;
-    if (tid < 4) s_cnt[tid] = 0;
+    if (tid < OCT_COUNTERS) s_cnt[tid] = 0;
     if (MODE == MODE_VR || MODE == MODE_LIGHT) {
         const float4 *g = reinterpret_cast<const float4 *>(a.tf_tables);
         const int nb = a.tf.nbins_max;
@@ -107,7 +108,7 @@ __global__ void __launch_bounds__(OBLOCK) octree_kernel(const ytgb_render_args a
         if (st.guarded) atomicAdd(&s_cnt[3], (unsigned long long)st.guarded);
         if (active) atomicAdd(&s_cnt[2], 1ull);
         __syncthreads();
-        if (tid < 4 && s_cnt[tid]) atomicAdd(a.counters + tid, s_cnt[tid]);
+        if (tid < OCT_COUNTERS && s_cnt[tid]) atomicAdd(a.counters + tid, s_cnt[tid]);
     }
 }
 
@@ -224,7 +225,8 @@ int octree_checks(const ytgb_render_args *a, const ytgb_octree_args *o, bool tra
 template <int MODE, int CTF>
 int octree_launch(const ytgb_render_args *a, const ytgb_octree_args *o, size_t smem, const Scratch &w,
                   cudaStream_t s, unsigned long long *h, long long *c) {
-    if (smem > 48 * 1024) {
+    // (static and dynamic shared memory together need the opt-in past 48 KB)
+    if (smem + OCT_COUNTERS * sizeof(unsigned long long) > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(octree_kernel<MODE, CTF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
         if (e != cudaSuccess) {
