@@ -255,49 +255,6 @@ YTGB_HD void step_advance(AxisStep &s, double d) {
     step_prepare(s, d);
 }
 
-// a / b, correctly rounded, on the integer pipe: about sixty instructions where
-// the float64 division takes ten of the float64 pipe's at 64 cycles each.  The
-// quotient of the 53-bit mantissas from a float32 reciprocal improved by
-// Newton's iteration in fixed point (two terms of the series), then its exact
-// remainder: every product below is needed modulo 2^64 only, since 2^83 and 2^105
-// vanish there and the differences formed are below 2^63.  An exact half does
-// not occur in a quotient of two numbers of one precision.  Zero, subnormal,
-// infinite and NaN operands and results near them take the division itself.
-YTGB_HD double quotient(double a, double b) {
-    const unsigned long long ab = (unsigned long long)dbits(a), bb = (unsigned long long)dbits(b);
-    const int ea = (int)(ab >> 52) & 0x7ff, eb = (int)(bb >> 52) & 0x7ff, e = ea - eb + 1022;
-    if ((unsigned)(ea - 1) > 2044u || (unsigned)(eb - 1) > 2044u || (unsigned)(e - 1) > 2043u) return ddiv(a, b);
-    const unsigned long long A = (ab & (unsigned long long)MANT52) | (1ull << 52),
-                             B = (bb & (unsigned long long)MANT52) | (1ull << 52);
-    // Y / 2^31 = 2^52 / B to 2^-22
-    const float y = frcp(ffrom(0x3f800000u | (unsigned)((B >> 29) & 0x7fffffu)));
-    const unsigned Y = (unsigned)fmul(y, 2147483648.0f);
-    // 2^83 - B Y = D, |D| < 2^62: 2^105 / B = 2^22 Y (1 + D / 2^83 + (D / 2^83)^2 + ...), to a few units
-    const long long D = -(long long)(B * Y);
-    const long long d = D >> 30;
-    const long long z1 = ((long long)Y * d) >> 31, z2 = (z1 * d) >> 53;
-    const unsigned long long Z = ((unsigned long long)Y << 22) + (unsigned long long)(z1 + z2);
-    const int k = A < B ? 53 : 52;  // the quotient A 2^k / B lies in [2^52, 2^53)
-#ifdef __CUDA_ARCH__
-    unsigned long long q = __umul64hi(A << 11, Z << 10) >> (62 - k);
-#else
-    unsigned long long q = (unsigned long long)(((unsigned __int128)(A << 11) * (Z << 10)) >> 64) >> (62 - k);
-#endif
-    long long R = (long long)((A << k) - q * B);
-    const long long Bs = (long long)B;
-    while (R < 0) {
-        R += Bs;
-        q--;
-    }
-    while (R >= Bs) {
-        R -= Bs;
-        q++;
-    }
-    q += 2 * R > Bs ? 1 : 0;
-    return dfrom((long long)(((ab ^ bb) & 0x8000000000000000ull) +
-                             ((unsigned long long)(e + (k == 52 ? 1 : 0) - 1) << 52) + q));
-}
-
 struct Ray {
     double pos[3];
     double dir[3];
