@@ -1003,13 +1003,14 @@ constexpr int V_REF = 2;
 // across one kernel: the AMR frame 1.36 -> 1.43 ms, 16 views in a batch 4.5 ->
 // 5.1 ms).  The batch kernel takes such walks through the loop with every test
 // in every step: with sample_many inlined for the light source or other table
-// sets, a build of it at 128 registers met an illegal address whose cause
-// reading did not show.
+// sets, a build of it at 128 registers met an illegal address whose cause was
+// not found.  The same function runs in the single-view kernels; on the CPU both
+// loops read nothing outside exactly sized arrays, in every form.
 constexpr int V_MANY = 4;
-#ifdef __CUDACC__
+#if defined(__CUDACC__) || defined(YTGB_GENERAL_LOOP)
 constexpr bool MANY_ALWAYS = false;
 #else
-constexpr bool MANY_ALWAYS = true;  // the test harness takes every walk through it
+constexpr bool MANY_ALWAYS = true;  // the test harness takes every walk through it, unless built for the batch's loop
 #endif
 
 // The variant a render's arguments call for: float64 range decisions where
