@@ -1,0 +1,92 @@
+"""The same images at another register budget, for the single-view kernels that
+the library compiles for 4 resident blocks per SM (128 registers a thread):
+several samples per cell, masked bricks, the light source, other table sets,
+and float64 range decisions.
+
+tests/test_gpu_codegen.py compares the library with a build at 4 blocks, which
+for these kernels is the library's own budget; here the second build is at 5 (96
+registers), which differs from every one of them."""
+import ctypes as C
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+import torch
+
+from test_gpu_batch import cams, mv_tf, same_bits
+from test_gpu_codegen import CSRC, ROOT
+from test_kernel_host import near_bound_case
+from yt_gb300 import _lib, testing, workloads
+from yt_gb300.amr_kdtree import AMRKDTree
+from yt_gb300.camera import Camera
+from yt_gb300.render import Renderer
+from yt_gb300.volume import BrickSet
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def other(cuda, tmp_path_factory):
+    nvcc = os.environ.get("NVCC") or shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    d = tmp_path_factory.mktemp("ytgb_regs96")
+    common = ["-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off",
+              f"-I{ROOT / 'include'}", f"-I{CSRC}"]
+    arch = ["-gencode", "arch=compute_103a,code=sm_103a"]
+    subprocess.run([nvcc, *arch, "--fmad=false", "-DYTGB_MIN_BLOCKS=5", *common, "-c", str(CSRC / "ytgb_render.cu"),
+                    "-o", str(d / "r.o")], check=True)
+    subprocess.run([nvcc, *common, "-c", str(CSRC / "ytgb_host.cpp"), "-o", str(d / "h.o")], check=True)
+    so = d / "libytgb_regs96.so"
+    subprocess.run([nvcc, *arch, "-shared", "-o", str(so), str(d / "r.o"), str(d / "h.o"), "-lcudart", "-Xcompiler",
+                    "-pthread"], check=True)
+    V = C.CDLL(str(so))
+    for name, (res, args) in _lib.SIGNATURES.items():
+        fn = getattr(V, name, None)
+        if fn is not None:
+            fn.restype, fn.argtypes = res, args
+    return V
+
+
+def test_single_view_kernels_at_another_budget(cuda, other):
+    grids = testing.amr_blob_grids(root=32, levels=2, patch=8, seed=0)
+    kd = AMRKDTree(grids, log_field=False)
+    bricks = kd.bricks()
+    rng = np.random.default_rng(5)
+    masked = [(d, (rng.random(dims) < 0.8).astype(np.uint8), le, re, dims) for d, _, le, re, dims in bricks]
+    two = [([d[0], np.sqrt(np.abs(d[0]))], m, le, re, dims) for d, m, le, re, dims in bricks]
+    lo = float(min(np.min(d[0]) for d, *_ in bricks))
+    hi = float(max(np.max(d[0]) for d, *_ in bricks))
+    tf = workloads.color_tf((lo, hi), 4)
+    near, near_tf = near_bound_case()
+    plain = Renderer(bricks, tf, device=cuda, kdtree=kd)
+    mask = Renderer(masked, tf, device=cuda, kdtree=kd)
+    mv = Renderer(two, mv_tf(lo, hi), device=cuda, kdtree=kd)
+    ref_ctf = Renderer(BrickSet(near, device=cuda, with_lo=True), near_tf["ctf"], device=cuda)
+    ref_gen = Renderer(BrickSet(near, device=cuda, with_lo=True), near_tf["general"], device=cuda)
+    ref_amr = Renderer(BrickSet(bricks, device=cuda, with_lo=True), tf, device=cuda, kdtree=kd)
+    light = ((-0.3, 0.8, 0.2), (0.9, 0.5, 0.2, 1.0))
+    V, S, P = _lib.VOLUME_RENDER, _lib.LIGHT_SOURCE, _lib.INTERPOLATED_PROJECTION
+    cases = [(plain, V, 3), (mask, V, 1), (mask, V, 2), (mv, V, 1), (mv, V, 2), (plain, S, 1), (plain, S, 3), (mv, S, 2),
+             (plain, P, 2), (ref_ctf, V, 1), (ref_ctf, V, 3), (ref_ctf, S, 2), (ref_gen, V, 1), (ref_amr, V, 1)]
+    close = Camera((0.3, 0.6, -1.0), 0.5, 1.5, 48, lens_type="perspective")
+    work = [(r, cam, kind, ns) for r, kind, ns in cases for cam in [*cams(2, seed=3), close]]
+
+    def images():
+        out = [r.render(cam, kind=kind, n_samples=ns, light=light if kind == S else None)
+               for r, cam, kind, ns in work]
+        torch.cuda.synchronize()
+        for r, *_ in work:
+            r.check()
+        return out
+
+    want = images()
+    saved = _lib._lib
+    try:
+        _lib._lib = other
+        got = images()
+    finally:
+        _lib._lib = saved
+    for (r, cam, kind, ns), a, b in zip(work, want, got):
+        assert same_bits(a, b), (kind, ns)
+    assert all(float(torch.nan_to_num(a).abs().max()) > 0 for a in want)
