@@ -482,13 +482,14 @@ int ytgb_offaxis_depths(const double *o, const double *u, const double *v, const
 int ytgb_offaxis_cells(const ytgb_offaxis_args *args, int32_t *d_error, void *stream);
 
 /* The same from the stamps' summed-area tables, which a caller that projects
- * a view more than once keeps beside its stamps: (max_depth, nsx + 1, nsy + 1)
- * uint64 device values, written by ytgb_offaxis_sums for images of nx x ny
- * from stamps of unit sum as ytgb_offaxis_depths and its normalisation give
- * them, 0 where the mask is 0 (an all-zero level is fine). */
+ * a view more than once keeps beside its stamps: ytgb_offaxis_sums_bytes (host)
+ * bytes of device memory, 16-byte aligned, written by ytgb_offaxis_sums for
+ * images of nx x ny from stamps of unit sum as ytgb_offaxis_depths and its
+ * normalisation give them, 0 where the mask is 0 (an all-zero level is fine). */
+int ytgb_offaxis_sums_bytes(int32_t nsx, int32_t nsy, int32_t max_depth, int64_t *bytes);
 int ytgb_offaxis_sums(const double *d_stamp, int32_t nsx, int32_t nsy, int32_t max_depth, int32_t nx, int32_t ny,
-                      uint64_t *d_sums, void *stream);
-int ytgb_offaxis_cells_sums(const ytgb_offaxis_args *args, const uint64_t *d_sums, int32_t *d_error, void *stream);
+                      void *d_sums, void *stream);
+int ytgb_offaxis_cells_sums(const ytgb_offaxis_args *args, const void *d_sums, int32_t *d_error, void *stream);
 
 /* ---- host: AMR kd-tree --------------------------------------------------- */
 /* Replaces AMRKDTree's Tree.build (amr_kdtree.py:109-118) over

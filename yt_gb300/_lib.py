@@ -207,6 +207,7 @@ SIGNATURES = {
     "ytgb_octree_scratch": (C.c_int, [C.POINTER(View), C.c_int32, C.POINTER(C.c_int64)]),
     "ytgb_render_octree_scheduled": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p]),
     "ytgb_offaxis_cells": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p]),
+    "ytgb_offaxis_sums_bytes": (C.c_int, [C.c_int32] * 3 + [C.POINTER(C.c_int64)]),
     "ytgb_offaxis_sums": (C.c_int, [C.c_void_p] + [C.c_int32] * 5 + [C.c_void_p, C.c_void_p]),
     "ytgb_offaxis_cells_sums": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "ytgb_offaxis_depths": (C.c_int, [C.c_void_p] * 4 + [C.c_int32] * 3 + [C.c_void_p, C.c_void_p]),

@@ -366,15 +366,16 @@ __global__ void __launch_bounds__(OA_BLOCK) offaxis_kernel(const ytgb_offaxis_ar
 // summed-area table.  A pixel's mass is the difference of four such corners.
 // The subcell kernel above spends some 30 to 90 float64 operations on a pixel,
 // at 2 per SM and cycle its bound (float64 pipe 90 % busy); a corner takes
-// three products of 64-bit integers, on the integer pipe.
+// three products of integers, on the integer pipe.
 //
-// The table is in fixed point, modulo 2^64, in units of 2^-(62 + s) of the
-// stamp's unit sum (level_shift): only differences are used, and those that
-// occur (one subcell column's or row's sum, a pixel's mass) fit 64 bits, so
-// that they are exact; in float64 the corners' cancellation would cost a large
-// cell's pixels three digits.  Entries are rounded to half a unit and the
-// products down, so that a pixel is within four units: 2e-17 of a pixel's
-// share of the cell, at every level.
+// The table is in fixed point of 128 bits, modulo 2^128, in units of
+// 2^-(126 + s) of the stamp's unit sum (level_shift): only differences are
+// used, and those that occur (one subcell column's or row's sum, a pixel's
+// mass) fit, so that they are exact.  An entry keeps its 53 bits down to 2^-73
+// of the sum, a cut subcell's dv its own 53 bits at any size, and a product is
+// rounded down by less than a unit: a pixel of n subcells is within n / 2 + 12
+// units.  So a pixel that a cell only grazes is as exact as a whole one down to
+// 1e-20 of the stamp's sum (64 bits lost 1e-12 of pixels of 1e-5 of the largest).
 //
 // The subcell boundaries, their pixels and dv are formed by the reference's
 // float64 operations, once per pixel boundary and axis.  A warp takes a few cells,
@@ -382,26 +383,22 @@ __global__ void __launch_bounds__(OA_BLOCK) offaxis_kernel(const ytgb_offaxis_ar
 // lane per cell for what depends on the cell alone, then one lane per pixel
 // boundary of as many cells as the table in shared memory holds, then the
 // pixels cell by cell, lanes over the columns and groups of lanes over the rows.
-// Measured (197,000 cells of levels 5-9 at 1024^2, 38 pixels to 2): 5.17 ms by
-// the subcell kernel, 1.02 with 32 cells a batch and float64 products and
-// conversions, 0.93 with the conversions on the integer pipe, 0.83 with one
-// block per four batches (the scheduler evens out the last wave), 0.74 with 6
-// blocks per SM and 16 cells, 0.73 with the products on the integer pipe, 0.69
-// with 8 cells and 7 blocks (12 and 6: 0.70; 6 and 6: 0.71).  Now the float64
-// pipe (boundaries and their divisions) and the integer pipe are each about
-// 40 % busy and issue 55 %; with plain stores for the atomics it is no faster.
+// 197,000 cells of levels 5-9 at 1024^2 (38 pixels to 2): 5.17 ms by the subcell
+// kernel, 1.01 here (0.69 with 64 bits).  Bound by the integer pipe's products.
 constexpr int OS_CAP = 520;   // pixel boundaries held per warp: a cell of 258 pixels each way
 constexpr int OS_CELLS = 8;   // cells of a warp's batch
 constexpr int OS_WARPS = 4;
 constexpr int OS_BLOCKS = 7;  // resident blocks per SM: 72 registers
+
+typedef unsigned __int128 u128;
 
 // s of a level of jm x km subcells.  A row or column of subcells holds at
 // most sqrt(6) / min(jm, km) of the sum (the largest plane section of a cube
 // is sqrt(2) of a face, across a cube 1 / sqrt(3) of the stamp's width) and a
 // subcell 3 sqrt(3) / (jm km) (the cube's diagonal); the level is chosen with
 // fewer than 8 subcells per pixel along the longer image axis
-// (image_utilities.pyx:92-99).  So the former stay below 2^64 units and a
-// pixel, which may hold the whole sum, at most 2^62 (with a margin of 1.3 for
+// (image_utilities.pyx:92-99).  So the former stay below 2^128 units and a
+// pixel, which may hold the whole sum, at most 2^126 (with a margin of 1.3 for
 // the stamp's own discretisation).
 __device__ __forceinline__ int level_shift(int jm, int km, int nx, int ny) {
     const int lg = 31 - __clz(min(jm, km));
@@ -412,33 +409,50 @@ __device__ __forceinline__ int level_shift(int jm, int km, int nx, int ny) {
     return s;
 }
 
+// The table of level d holds (jm + 1) x (km + 1) sums, rows of km + 1, behind
+// those of the levels before it.
+__host__ __device__ __forceinline__ int level_extent(int ns, int depth) { return depth < 31 && (1 << depth) < ns ? 1 << depth : ns; }
+__host__ __device__ __forceinline__ long long level_offset(int nsx, int nsy, int depth) {
+    long long o = 0;
+    for (int d = 0; d < depth; d++) o += (long long)(level_extent(nsx, d) + 1) * (level_extent(nsy, d) + 1);
+    return o;
+}
+
 struct SplatCell {
     double x, y, dlx, dly, cq, cw;
     float bx, by, sx, sy;  // estimate of the subcell at a pixel boundary: ceil(s * P + b) - 1
     int depth, jm, km, unit;  // unit: 2^-unit is the table's
+    long long base;           // the level's first sum
     int P0, Pn, Q0, Qn;    // first pixel and number of pixels, per axis (0: nothing to do)
 };
 
 struct SplatSmem {
     SplatCell cell[OS_CELLS];
-    unsigned long long w[OS_CAP];  // dv of the cut subcell, 2^-64
+    unsigned long long w[OS_CAP];  // dv of the cut subcell (split_share)
     int at[OS_CAP];                // its index
     int off[OS_CELLS], who[OS_CELLS];          // the packed cells' first entries, and which cells they are
 };
 
-// floor(a b / 2^64)
-__device__ __forceinline__ unsigned long long scale64(unsigned long long a, unsigned long long b) {
-    return __umul64hi(a, b);
+// A dv in (0, 1) as its mantissa (1 at bit 63) and, in the low bits that its 53
+// leave free, the power of two it stands below 1; 0 for what is not above 0
+// (and below 2^-64, which no dv is: it is a difference of numbers of pixels).
+__device__ __forceinline__ unsigned long long split_share(double x) {
+    const long long b = dbits(x);
+    const int sh = 1022 - (int)(b >> 52);
+    if (b <= 0 || sh > 63) return 0ull;
+    return ((unsigned long long)((b & MANT52) | (1LL << 52)) << 11) | (unsigned)sh;
 }
 
-// x in [0, 1] in units of 2^-64 (1 as the largest value), anything else clipped
-__device__ __forceinline__ unsigned long long unit64(double x) {
-    const long long b = dbits(x);
-    if (b <= 0 || b > 0x7ff0000000000000LL) return 0ull;  // negative, zero, NaN
-    if (b >= 0x3ff0000000000000LL) return ~0ull;
-    const int sh = (int)(b >> 52) - 1011;  // x = m 2^(e - 1075)
-    const unsigned long long m = (unsigned long long)((b & MANT52) | (1LL << 52));
-    return sh >= 0 ? m << sh : (sh > -53 ? m >> -sh : 0ull);
+// floor(a w) of a split_share w
+__device__ __forceinline__ u128 scale_share(u128 a, unsigned long long w) {
+    const unsigned long long m = w & ~2047ull, hi = (unsigned long long)(a >> 64);
+    const u128 p = (u128)hi * m + __umul64hi((unsigned long long)a, m);
+    return p >> (int)(w & 63);
+}
+
+__device__ __forceinline__ u128 load_sum(const ulonglong2 *__restrict__ S, long long i) {
+    const ulonglong2 v = __ldg(S + i);
+    return ((u128)v.y << 64) | v.x;
 }
 
 // (double)v for 0 <= v < 2^31 and the truncation of |x| < 2^31 (others by the
@@ -492,7 +506,12 @@ __device__ __forceinline__ void cut_subcell(int P, int m, double d, double x, in
         e1 = truncate(b1);
     }
     at = j;
-    w = j < m && e0 <= P ? unit64(ytgb::ddiv(ytgb::dsub(to_double(e1), b0), ytgb::dsub(b1, b0))) : 0ull;
+    w = 0ull;
+    if (j < m && e0 <= P) {
+        const double dv = ytgb::ddiv(ytgb::dsub(to_double(e1), b0), ytgb::dsub(b1, b0));
+        if (dv >= 1.0) at = j + 1;  // the whole subcell is left of the boundary
+        else w = split_share(dv);
+    }
 }
 
 // A float64 factor as a 64-bit mantissa (1 at bit 63), exponent and sign, for
@@ -527,17 +546,22 @@ __device__ __forceinline__ double scaled_mass(unsigned long long m, int down, co
 
 // the table's value at a corner: rows at, at + 1 and columns b0, b1 (two
 // neighbours, or twice the last)
-__device__ __forceinline__ unsigned long long corner(const unsigned long long *__restrict__ S, int stride, int m,
-                                                     int at, unsigned long long wa, int b0, int b1,
-                                                     unsigned long long wb) {
-    const unsigned long long *r0 = S + (long long)at * stride, *r1 = S + (long long)min(at + 1, m) * stride;
-    const unsigned long long u0 = __ldg(r0 + b0), u1 = __ldg(r0 + b1), v0 = __ldg(r1 + b0), v1 = __ldg(r1 + b1);
-    const unsigned long long u = u0 + scale64(u1 - u0, wb), v = v0 + scale64(v1 - v0, wb);
-    return u + scale64(v - u, wa);
+__device__ __forceinline__ u128 corner(const ulonglong2 *__restrict__ S, int stride, int m, int at,
+                                       unsigned long long wa, int b0, int b1, unsigned long long wb) {
+    const ulonglong2 *r0 = S + (long long)at * stride, *r1 = S + (long long)min(at + 1, m) * stride;
+    const u128 u0 = load_sum(r0, b0), u1 = load_sum(r0, b1), v0 = load_sum(r1, b0), v1 = load_sum(r1, b1);
+    const u128 u = u0 + scale_share(u1 - u0, wb), v = v0 + scale_share(v1 - v0, wb);
+    return u + scale_share(v - u, wa);
+}
+
+__device__ __forceinline__ u128 shuffle_up(u128 v, int d) {
+    const unsigned long long lo = __shfl_up_sync(0xffffffffu, (unsigned long long)v, d);
+    const unsigned long long hi = __shfl_up_sync(0xffffffffu, (unsigned long long)(v >> 64), d);
+    return ((u128)hi << 64) | lo;
 }
 
 __global__ void __launch_bounds__(OS_WARPS * 32, OS_BLOCKS)
-splat_kernel(const ytgb_offaxis_args a, const unsigned long long *__restrict__ sums, int32_t *error) {
+splat_kernel(const ytgb_offaxis_args a, const ulonglong2 *__restrict__ sums, int32_t *error) {
     __shared__ SplatSmem s_all[OS_WARPS];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     SplatSmem &sm = s_all[wib];
@@ -547,7 +571,6 @@ splat_kernel(const ytgb_offaxis_args a, const unsigned long long *__restrict__ s
     const double sq3x4 = ytgb::dmul(4.0, sq3);
     const double nmax = nx > ny ? (double)nx : (double)ny;  // fmax(Nx, Ny)
     const long long batches = (a.n + OS_CELLS - 1) / OS_CELLS;
-    const int stride = a.nsy + 1;
     for (long long bt = (long long)blockIdx.x * OS_WARPS + wib; bt < batches; bt += (long long)gridDim.x * OS_WARPS) {
         // ---- one lane per cell
         const long long c = bt + (long long)lane * batches;
@@ -593,7 +616,8 @@ splat_kernel(const ytgb_offaxis_args a, const unsigned long long *__restrict__ s
                     sc.depth = depth;
                     sc.jm = jm;
                     sc.km = km;
-                    sc.unit = 62 + level_shift(jm, km, nx, ny);
+                    sc.unit = 126 + level_shift(jm, km, nx, ny);
+                    sc.base = level_offset(a.nsx, a.nsy, depth);
                     // pixels the cell can reach (the boundaries are nondecreasing)
                     const int P0 = max(__double2int_rz(boundary(0, jm, sc.dlx, x, nx)), 0);
                     const int P1 = min(__double2int_rz(boundary(jm, jm, sc.dlx, x, nx)), nx - 1);
@@ -668,8 +692,8 @@ splat_kernel(const ytgb_offaxis_args a, const unsigned long long *__restrict__ s
             // ---- the pixels, cell by cell
             for (int i = 0; i < n_take; i++) {
                 const SplatCell &sc = sm.cell[sm.who[i]];
-                const int o = sm.off[i], rows = sc.Pn, jm = sc.jm, km = sc.km;
-                const unsigned long long *S = sums + (long long)sc.depth * (a.nsx + 1) * stride;
+                const int o = sm.off[i], rows = sc.Pn, jm = sc.jm, km = sc.km, stride = km + 1;
+                const ulonglong2 *S = sums + sc.base;
                 const Factor fq = factor_of(sc.cq), fw = factor_of(sc.cw);
                 const bool plain = fq.ok && fw.ok;
                 const int *ra = sm.at + o, *ca = ra + rows + 1;
@@ -687,26 +711,27 @@ splat_kernel(const ytgb_offaxis_args a, const unsigned long long *__restrict__ s
                     const int steps = (rows + groups - 1) / groups;
                     const int Q = sc.Q0 + q - 1;  // the pixel left of this boundary
                     const bool px = on && lane > g * nb;
-                    unsigned long long prev = on ? corner(S, stride, jm, ra[r0], rw[r0], b, b1, wb) : 0ull;
+                    u128 prev = on ? corner(S, stride, jm, ra[r0], rw[r0], b, b1, wb) : (u128)0;
                     for (int k = 0; k < steps; k++) {
                         const int r = min(r0 + k + 1, r1);
-                        const unsigned long long G = on ? corner(S, stride, jm, ra[r], rw[r], b, b1, wb) : 0ull;
-                        const unsigned long long d = G - prev;
+                        const u128 G = on ? corner(S, stride, jm, ra[r], rw[r], b, b1, wb) : (u128)0;
+                        const u128 d = G - prev;
                         prev = G;
-                        const unsigned long long dl = __shfl_up_sync(0xffffffffu, d, 1);
-                        const long long mass = (long long)(d - dl);  // (rounding may leave a few units below 0)
+                        const __int128 mass = (__int128)(d - shuffle_up(d, 1));  // (rounding may leave a few units below 0)
                         if (px && r0 + k < r1 && mass > 0) {
                             const long long idx = (long long)(sc.P0 + r0 + k) * nx + Q;
                             if (idx < npix) {
-                                const int sh = __clzll(mass);
-                                const unsigned long long m = (unsigned long long)mass << sh;
-                                const int down = sc.unit - 63 + sh;
+                                // the mass' upper 64 bits from its first 1
+                                const unsigned long long mh = (unsigned long long)(mass >> 64);
+                                const int sh = mh ? __clzll((long long)mh) : 64 + __clzll((long long)mass);
+                                const unsigned long long m = (unsigned long long)(((u128)mass << sh) >> 64);
+                                const int down = sc.unit - 127 + sh;
                                 double vq, vw;
                                 if (plain) {
                                     vq = scaled_mass(m, down, fq);
                                     vw = scaled_mass(m, down, fw);
                                 } else {
-                                    const double f = dfrom(dbits((double)mass) - ((long long)sc.unit << 52));
+                                    const double f = dfrom(dbits((double)m) - ((long long)(down + 63) << 52));
                                     vq = ytgb::dmul(f, sc.cq);
                                     vw = ytgb::dmul(f, sc.cw);
                                 }
@@ -724,26 +749,46 @@ splat_kernel(const ytgb_offaxis_args a, const unsigned long long *__restrict__ s
     }
 }
 
+// a stamp entry in units of 2^-unit (to nearest; 0 where it is not above 0)
+__device__ __forceinline__ u128 stamp_units(double x, int unit) {
+    const long long b = dbits(x);
+    const int e = (int)(b >> 52);
+    if (b <= 0 || e >= 0x7ff) return 0;
+    const u128 m = (u128)(unsigned long long)((b & MANT52) | (e > 0 ? 1LL << 52 : 0LL));
+    const int sh = (e > 0 ? e : 1) - 1075 + unit;
+    if (sh >= 0) return sh < 128 ? m << sh : (u128)0;
+    return sh > -64 ? (m + ((u128)1 << (-sh - 1))) >> -sh : (u128)0;
+}
+
+__device__ __forceinline__ void store_sum(ulonglong2 *S, long long i, u128 v) {
+    S[i] = make_ulonglong2((unsigned long long)v, (unsigned long long)(v >> 64));
+}
+
 // The summed-area table of one stamp level per block: rows, then columns.
 __global__ void __launch_bounds__(256)
-sums_kernel(const double *stamp, int nsx, int nsy, int nx, int ny, unsigned long long *sums) {
+sums_kernel(const double *stamp, int nsx, int nsy, int nx, int ny, ulonglong2 *sums) {
     const int depth = blockIdx.x;
-    const int jm = depth < 31 ? min(nsx, 1 << depth) : nsx, km = depth < 31 ? min(nsy, 1 << depth) : nsy;
+    const int jm = level_extent(nsx, depth), km = level_extent(nsy, depth), stride = km + 1;
     const double *st = stamp + (long long)depth * nsx * nsy;
-    const double unit = dfrom((long long)(1023 + 62 + level_shift(jm, km, nx, ny)) << 52);
-    const long long stride = nsy + 1;
-    unsigned long long *S = sums + (long long)depth * (nsx + 1) * stride;
+    const int unit = 126 + level_shift(jm, km, nx, ny);
+    ulonglong2 *S = sums + level_offset(nsx, nsy, depth);
     for (int j = threadIdx.x; j <= jm; j += 256) {
-        unsigned long long acc = 0;
-        S[j * stride] = 0;
+        u128 acc = 0;
+        store_sum(S, (long long)j * stride, 0);
         for (int k = 0; k < km; k++) {
-            if (j > 0) acc += __double2ull_rn(ytgb::dmul(__ldg(st + (long long)(j - 1) * nsy + k), unit));
-            S[j * stride + k + 1] = acc;
+            if (j > 0) acc += stamp_units(__ldg(st + (long long)(j - 1) * nsy + k), unit);
+            store_sum(S, (long long)j * stride + k + 1, acc);
         }
     }
     __syncthreads();
-    for (int k = threadIdx.x; k <= km; k += 256)
-        for (int j = 1; j <= jm; j++) S[j * stride + k] += S[(j - 1) * stride + k];
+    for (int k = threadIdx.x; k <= km; k += 256) {
+        u128 acc = 0;
+        for (int j = 0; j <= jm; j++) {
+            const ulonglong2 v = S[(long long)j * stride + k];
+            acc += ((u128)v.y << 64) | v.x;
+            store_sum(S, (long long)j * stride + k, acc);
+        }
+    }
 }
 
 }  // namespace
@@ -792,15 +837,24 @@ extern "C" int ytgb_offaxis_cells(const ytgb_offaxis_args *args, int32_t *d_erro
     return YTGB_OK;
 }
 
+extern "C" int ytgb_offaxis_sums_bytes(int32_t nsx, int32_t nsy, int32_t max_depth, int64_t *bytes) {
+    if (!bytes || nsx < 1 || nsy < 1 || max_depth < 2 || max_depth > 30) {
+        ytgb_set_error("ytgb_offaxis_sums_bytes: null argument or bad sizes");
+        return YTGB_ERR_INVALID;
+    }
+    *bytes = (int64_t)sizeof(ulonglong2) * level_offset(nsx, nsy, max_depth);
+    return YTGB_OK;
+}
+
 extern "C" int ytgb_offaxis_sums(const double *d_stamp, int32_t nsx, int32_t nsy, int32_t max_depth, int32_t nx,
-                                 int32_t ny, uint64_t *d_sums, void *stream) {
-    if (!d_stamp || !d_sums || ((uintptr_t)d_stamp & 7) || ((uintptr_t)d_sums & 7) || nsx < 1 || nsy < 1 ||
+                                 int32_t ny, void *d_sums, void *stream) {
+    if (!d_stamp || !d_sums || ((uintptr_t)d_stamp & 7) || ((uintptr_t)d_sums & 15) || nsx < 1 || nsy < 1 ||
         max_depth < 2 || max_depth > 30 || nx < 1 || ny < 1) {
         ytgb_set_error("ytgb_offaxis_sums: null or misaligned array, or bad sizes");
         return YTGB_ERR_INVALID;
     }
     sums_kernel<<<max_depth, 256, 0, (cudaStream_t)stream>>>(d_stamp, nsx, nsy, nx, ny,
-                                                             reinterpret_cast<unsigned long long *>(d_sums));
+                                                             reinterpret_cast<ulonglong2 *>(d_sums));
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         ytgb_set_error(std::string("ytgb_offaxis_sums: ") + cudaGetErrorString(e));
@@ -809,11 +863,11 @@ extern "C" int ytgb_offaxis_sums(const double *d_stamp, int32_t nsx, int32_t nsy
     return YTGB_OK;
 }
 
-extern "C" int ytgb_offaxis_cells_sums(const ytgb_offaxis_args *args, const uint64_t *d_sums, int32_t *d_error,
+extern "C" int ytgb_offaxis_cells_sums(const ytgb_offaxis_args *args, const void *d_sums, int32_t *d_error,
                                        void *stream) {
     if (int st = offaxis_checks(args, d_error)) return st;
     const ytgb_offaxis_args &a = *args;
-    if (!d_sums || ((uintptr_t)d_sums & 7)) {
+    if (!d_sums || ((uintptr_t)d_sums & 15)) {
         ytgb_set_error("ytgb_offaxis_cells_sums: null or misaligned table of sums");
         return YTGB_ERR_INVALID;
     }
@@ -821,7 +875,7 @@ extern "C" int ytgb_offaxis_cells_sums(const ytgb_offaxis_args *args, const uint
     const long long batches = (a.n + OS_CELLS - 1) / OS_CELLS;
     const int blocks = (int)std::min<long long>((batches + OS_WARPS - 1) / OS_WARPS, 1 << 20);
     splat_kernel<<<blocks, OS_WARPS * 32, 0, (cudaStream_t)stream>>>(
-        a, reinterpret_cast<const unsigned long long *>(d_sums), d_error);
+        a, reinterpret_cast<const ulonglong2 *>(d_sums), d_error);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         ytgb_set_error(std::string("ytgb_offaxis_cells_sums: ") + cudaGetErrorString(e));

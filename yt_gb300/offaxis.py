@@ -118,10 +118,13 @@ def _device_sums(stamp, shape, nx, ny):
     """The stamps' summed-area tables (``ytgb_offaxis_sums``), complete when
     returned (a projection may run on another stream)."""
     max_depth, nsx, nsy = shape
-    sums = torch.empty(max_depth * (nsx + 1) * (nsy + 1), dtype=torch.int64, device=stamp.device)
+    L = _lib.lib()
+    size = C.c_int64()
+    _lib.check(L.ytgb_offaxis_sums_bytes(nsx, nsy, max_depth, C.byref(size)), "ytgb_offaxis_sums_bytes")
+    sums = torch.empty(size.value, dtype=torch.uint8, device=stamp.device)
     s = torch.cuda.current_stream(stamp.device)
-    _lib.check(_lib.lib().ytgb_offaxis_sums(stamp.data_ptr(), nsx, nsy, max_depth, nx, ny, sums.data_ptr(),
-                                            C.c_void_p(s.cuda_stream)), "ytgb_offaxis_sums")
+    _lib.check(L.ytgb_offaxis_sums(stamp.data_ptr(), nsx, nsy, max_depth, nx, ny, sums.data_ptr(),
+                                   C.c_void_p(s.cuda_stream)), "ytgb_offaxis_sums")
     s.synchronize()
     return sums
 
