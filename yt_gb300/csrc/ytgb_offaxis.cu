@@ -749,6 +749,14 @@ splat_kernel(const ytgb_offaxis_args a, const ulonglong2 *__restrict__ sums, int
     }
 }
 
+// ---- the summed-area tables: rows, then columns ------------------------------
+// One warp per row of a level, lanes along it; then one block per level and 32
+// columns, each warp adding up a run of rows: every access is a warp's 512
+// contiguous bytes.  A view's tables for cells of 0.15 and 0.3 of a 1024^2 image:
+// 644 and 2139 us with one block per level and a thread per row, now 56 and 78
+// (36 of them the launches, the allocation and the wait).
+constexpr int SR_WARPS = 4, SC_WARPS = 16;
+
 // a stamp entry in units of 2^-unit (to nearest; 0 where it is not above 0)
 __device__ __forceinline__ u128 stamp_units(double x, int unit) {
     const long long b = dbits(x);
@@ -764,31 +772,59 @@ __device__ __forceinline__ void store_sum(ulonglong2 *S, long long i, u128 v) {
     S[i] = make_ulonglong2((unsigned long long)v, (unsigned long long)(v >> 64));
 }
 
-// The summed-area table of one stamp level per block: rows, then columns.
-__global__ void __launch_bounds__(256)
-sums_kernel(const double *stamp, int nsx, int nsy, int nx, int ny, ulonglong2 *sums) {
-    const int depth = blockIdx.x;
-    const int jm = level_extent(nsx, depth), km = level_extent(nsy, depth), stride = km + 1;
-    const double *st = stamp + (long long)depth * nsx * nsy;
+__global__ void __launch_bounds__(SR_WARPS * 32)
+sum_rows_kernel(const double *stamp, int nsx, int nsy, int nx, int ny, ulonglong2 *sums) {
+    const int depth = blockIdx.y, lane = threadIdx.x & 31;
+    const int jm = level_extent(nsx, depth), km = level_extent(nsy, depth);
+    const int j = blockIdx.x * SR_WARPS + (threadIdx.x >> 5);  // the sums' row: 0 is empty
+    if (j > jm) return;
+    ulonglong2 *row = sums + level_offset(nsx, nsy, depth) + (long long)j * (km + 1);
+    const double *st = stamp + ((long long)depth * nsx + (j - 1)) * nsy;
     const int unit = 126 + level_shift(jm, km, nx, ny);
-    ulonglong2 *S = sums + level_offset(nsx, nsy, depth);
-    for (int j = threadIdx.x; j <= jm; j += 256) {
-        u128 acc = 0;
-        store_sum(S, (long long)j * stride, 0);
-        for (int k = 0; k < km; k++) {
-            if (j > 0) acc += stamp_units(__ldg(st + (long long)(j - 1) * nsy + k), unit);
-            store_sum(S, (long long)j * stride + k + 1, acc);
+    u128 before = 0;
+    if (lane == 0) store_sum(row, 0, 0);
+    for (int k0 = 0; k0 < km; k0 += 32) {
+        const int k = k0 + lane;
+        u128 v = j > 0 && k < km ? stamp_units(__ldg(st + k), unit) : (u128)0;
+        for (int d = 1; d < 32; d <<= 1) {
+            const u128 u = shuffle_up(v, d);
+            if (lane >= d) v += u;
         }
+        v += before;
+        if (k < km) store_sum(row, k + 1, v);
+        const unsigned long long lo = __shfl_sync(0xffffffffu, (unsigned long long)v, 31);
+        const unsigned long long hi = __shfl_sync(0xffffffffu, (unsigned long long)(v >> 64), 31);
+        before = ((u128)hi << 64) | lo;
     }
-    __syncthreads();
-    for (int k = threadIdx.x; k <= km; k += 256) {
-        u128 acc = 0;
-        for (int j = 0; j <= jm; j++) {
-            const ulonglong2 v = S[(long long)j * stride + k];
+}
+
+__global__ void __launch_bounds__(SC_WARPS * 32) sum_columns_kernel(int nsx, int nsy, ulonglong2 *sums) {
+    __shared__ ulonglong2 part[SC_WARPS][32];
+    const int depth = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int jm = level_extent(nsx, depth), stride = level_extent(nsy, depth) + 1;
+    const int k = blockIdx.x * 32 + lane;
+    if ((int)blockIdx.x * 32 >= stride) return;  // (the whole block)
+    ulonglong2 *col = sums + level_offset(nsx, nsy, depth) + k;
+    const int per = (jm + SC_WARPS) / SC_WARPS;  // of jm + 1 rows
+    const int j0 = min(warp * per, jm + 1), j1 = min(j0 + per, jm + 1);
+    u128 acc = 0;
+    if (k < stride)
+#pragma unroll 4
+        for (int j = j0; j < j1; j++) {
+            const ulonglong2 v = col[(long long)j * stride];
             acc += ((u128)v.y << 64) | v.x;
-            store_sum(S, (long long)j * stride + k, acc);
         }
-    }
+    part[warp][lane] = make_ulonglong2((unsigned long long)acc, (unsigned long long)(acc >> 64));
+    __syncthreads();
+    acc = 0;
+    for (int w = 0; w < warp; w++) acc += ((u128)part[w][lane].y << 64) | part[w][lane].x;
+    if (k < stride)
+#pragma unroll 4
+        for (int j = j0; j < j1; j++) {
+            const ulonglong2 v = col[(long long)j * stride];
+            acc += ((u128)v.y << 64) | v.x;
+            store_sum(col, (long long)j * stride, acc);
+        }
 }
 
 }  // namespace
@@ -853,8 +889,11 @@ extern "C" int ytgb_offaxis_sums(const double *d_stamp, int32_t nsx, int32_t nsy
         ytgb_set_error("ytgb_offaxis_sums: null or misaligned array, or bad sizes");
         return YTGB_ERR_INVALID;
     }
-    sums_kernel<<<max_depth, 256, 0, (cudaStream_t)stream>>>(d_stamp, nsx, nsy, nx, ny,
-                                                             reinterpret_cast<ulonglong2 *>(d_sums));
+    const int jm = level_extent(nsx, max_depth - 1), km = level_extent(nsy, max_depth - 1);  // the largest level
+    sum_rows_kernel<<<dim3(jm / SR_WARPS + 1, max_depth), SR_WARPS * 32, 0, (cudaStream_t)stream>>>(
+        d_stamp, nsx, nsy, nx, ny, reinterpret_cast<ulonglong2 *>(d_sums));
+    sum_columns_kernel<<<dim3(km / 32 + 1, max_depth), SC_WARPS * 32, 0, (cudaStream_t)stream>>>(
+        nsx, nsy, reinterpret_cast<ulonglong2 *>(d_sums));
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         ytgb_set_error(std::string("ytgb_offaxis_sums: ") + cudaGetErrorString(e));
