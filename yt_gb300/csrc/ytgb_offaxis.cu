@@ -379,10 +379,11 @@ __global__ void __launch_bounds__(OA_BLOCK) offaxis_kernel(const ytgb_offaxis_ar
 //
 // The subcell boundaries, their pixels and dv are formed by the reference's
 // float64 operations, once per pixel boundary and axis.  A warp takes a few cells,
-// strided over the list so that each batch has cells of all sizes: first one
-// lane per cell for what depends on the cell alone, then one lane per pixel
-// boundary of as many cells as the table in shared memory holds, then the
-// pixels cell by cell, lanes over the columns and groups of lanes over the rows.
+// strided over the list so that each batch has cells of all sizes (one where there
+// are no more cells than warps): first one lane per cell for what depends on the
+// cell alone, then one lane per pixel boundary of as many cells as the table in
+// shared memory holds, then the pixels cell by cell, lanes over the columns and
+// groups of lanes over the rows.
 // 197,000 cells of levels 5-9 at 1024^2 (38 pixels to 2): 5.17 ms by the subcell
 // kernel, 1.01 here (0.69 with 64 bits).  Bound by the integer pipe's products.
 constexpr int OS_CAP = 520;   // pixel boundaries held per warp: a cell of 258 pixels each way
@@ -561,7 +562,7 @@ __device__ __forceinline__ u128 shuffle_up(u128 v, int d) {
 }
 
 __global__ void __launch_bounds__(OS_WARPS * 32, OS_BLOCKS)
-splat_kernel(const ytgb_offaxis_args a, const ulonglong2 *__restrict__ sums, int32_t *error) {
+splat_kernel(const ytgb_offaxis_args a, const ulonglong2 *__restrict__ sums, long long batches, int32_t *error) {
     __shared__ SplatSmem s_all[OS_WARPS];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     SplatSmem &sm = s_all[wib];
@@ -570,7 +571,6 @@ splat_kernel(const ytgb_offaxis_args a, const ulonglong2 *__restrict__ sums, int
     const double sq3 = ytgb::dsqrt(3.0);
     const double sq3x4 = ytgb::dmul(4.0, sq3);
     const double nmax = nx > ny ? (double)nx : (double)ny;  // fmax(Nx, Ny)
-    const long long batches = (a.n + OS_CELLS - 1) / OS_CELLS;
     for (long long bt = (long long)blockIdx.x * OS_WARPS + wib; bt < batches; bt += (long long)gridDim.x * OS_WARPS) {
         // ---- one lane per cell
         const long long c = bt + (long long)lane * batches;
@@ -911,10 +911,14 @@ extern "C" int ytgb_offaxis_cells_sums(const ytgb_offaxis_args *args, const void
         return YTGB_ERR_INVALID;
     }
     if (a.n == 0) return YTGB_OK;
-    const long long batches = (a.n + OS_CELLS - 1) / OS_CELLS;
+    // a warp takes a second cell only where there are more cells than resident warps:
+    // in batches of OS_CELLS fewer cells left most of the chip idle (1,000 cells of
+    // 111 pixels 1.92 ms, now 0.29)
+    const long long resident = (long long)offaxis_blocks(1ll << 40, OS_BLOCKS) * OS_WARPS;
+    const long long batches = std::max<long long>((a.n + OS_CELLS - 1) / OS_CELLS, std::min<long long>(a.n, resident));
     const int blocks = (int)std::min<long long>((batches + OS_WARPS - 1) / OS_WARPS, 1 << 20);
     splat_kernel<<<blocks, OS_WARPS * 32, 0, (cudaStream_t)stream>>>(
-        a, reinterpret_cast<const ulonglong2 *>(d_sums), d_error);
+        a, reinterpret_cast<const ulonglong2 *>(d_sums), batches, d_error);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         ytgb_set_error(std::string("ytgb_offaxis_cells_sums: ") + cudaGetErrorString(e));

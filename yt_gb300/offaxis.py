@@ -11,7 +11,7 @@ spread bilinearly over the pixels it overlaps.
 :func:`offaxis_stamp` computes the stamps on the host exactly as the
 reference does (the same float64 operations, vectorised with numpy);
 :class:`CellSplat` keeps the cells resident on the device and runs the
-``ytgb_offaxis_cells_sums`` launch; :func:`add_cells_to_image_offaxis` is the
+``ytgb_offaxis_cells_sums`` launch (``ytgb_offaxis_cells`` for few cells); :func:`add_cells_to_image_offaxis` is the
 drop-in with the reference's keyword signature, and
 :func:`project_cells` restates the driver's steps around it (recentring,
 periodic wrap, scaling by the image width, the final ``wmax / sqrt(3)``).
@@ -129,6 +129,14 @@ def _device_sums(stamp, shape, nx, ny):
     return sums
 
 
+# Up to this many cells are projected by ytgb_offaxis_cells, straight from the
+# stamps: a warp has one cell then, and a projection takes as long either way (us,
+# subcells / sums: 1,024 cells of 2 pixels 15 / 15, of 17 33 / 35, of 64 316 / 294;
+# 2,048 23 / 23, 52 / 54, 515 / 447; 4,096 35 / 33, 107 / 78, 1205 / 717), while a
+# new view pays 36 us for its sums.
+FEW_CELLS = 2048
+
+
 class CellSplat:
     """Cells resident on the device for repeated off-axis projections.
 
@@ -159,7 +167,8 @@ class CellSplat:
         key = (rotation.tobytes(), nx, ny, npix_min)
         if key not in self._stamps:
             stamp, shape = _device_stamp(rotation, self.dx_max, nx, ny, npix_min, self.device)
-            self._sums[key] = _device_sums(stamp, shape, nx, ny)
+            if self.n > FEW_CELLS:
+                self._sums[key] = _device_sums(stamp, shape, nx, ny)
             self._stamps[key] = stamp, shape
         return self._stamps[key]
 
@@ -189,6 +198,10 @@ class CellSplat:
         a.n, a.nx, a.ny, a.nsx, a.nsy, a.max_depth = self.n, nx, ny, nsx, nsy, max_depth
         s = stream or torch.cuda.current_stream(self.device)
         err = None if error is None else error.data_ptr()
+        if self.n <= FEW_CELLS:
+            _lib.check(_lib.lib().ytgb_offaxis_cells(C.byref(a), C.c_void_p(err), C.c_void_p(s.cuda_stream)),
+                       "ytgb_offaxis_cells")
+            return out
         sums = self._sums[(rotation.tobytes(), nx, ny, npix_min)]
         _lib.check(_lib.lib().ytgb_offaxis_cells_sums(C.byref(a), sums.data_ptr(), C.c_void_p(err),
                                                       C.c_void_p(s.cuda_stream)), "ytgb_offaxis_cells_sums")
