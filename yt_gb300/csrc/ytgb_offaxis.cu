@@ -742,6 +742,19 @@ splat_kernel(const ytgb_offaxis_args a, const ulonglong2 *__restrict__ sums, lon
                     }
                 }
             }
+            // a quantity or weight that is not finite reaches every pixel of its cell's
+            // rectangle, also those of no mass, as in the subcell kernel
+            for (int i = 0; i < n_take; i++) {
+                const SplatCell &sc = sm.cell[sm.who[i]];
+                if (isfinite(sc.cq) && isfinite(sc.cw)) continue;
+                for (long long t = lane; t < (long long)sc.Pn * sc.Qn; t += 32) {
+                    const long long idx = (sc.P0 + t / sc.Qn) * nx + sc.Q0 + t % sc.Qn;
+                    if (idx < npix) {
+                        atomicAdd(a.buffer + idx, ytgb::dmul(0.0, sc.cq));
+                        atomicAdd(a.buffer_weight + idx, ytgb::dmul(0.0, sc.cw));
+                    }
+                }
+            }
             __syncwarp();  // the tables are rewritten
             left &= ~take;
         }
