@@ -51,7 +51,10 @@ extern "C" {
 
 /* render flags */
 #define YTGB_FLAG_NO_COMPENSATION 1u   /* plain FP32 accumulation (precision study) */
-#define YTGB_FLAG_TILE_SHIFT 8         /* bits 8..11: tile shape 0 = 8x16, 1 = 16x8, 2 = 4x32 pixels */
+#define YTGB_FLAG_TILE_SHIFT 8         /* bits 8..11: tile shape 0 = 8x16, 1 = 16x8, 2 = 4x32 pixels (the image
+                                        * is the same in each).  A request: single-view launches with several
+                                        * samples per cell, masks, the light source or tables other than a
+                                        * ColorTransferFunction's take 16x8 */
 
 /* One brick: the fields of yt's VolumeContainer (volume_container.pxd:13-33,
  * filled by PartitionedGrid.__cinit__, partitioned_grid.pyx:28-63), plus

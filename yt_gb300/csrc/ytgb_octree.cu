@@ -27,17 +27,11 @@ constexpr int OCT_COUNTERS = 4;
 
 static_assert(sizeof(ytgb_onode) == sizeof(ONode), "ytgb_onode layout");
 
-// Bound by the integer pipe (55 % busy, the traversal's selects and 64-bit
+// Bound by the integer pipe (57 % busy, the traversal's selects and 64-bit
 // comparisons) and by lanes waiting for each other (22 of 32 active), with the
-// float64 pipe at 37 %.  1024^2 frame of a 197,000-cell octree of levels 5-9,
-// ms: 2.98 with float64 midpoints and conversions, whole 80-byte frames on the
-// stack and each cell sampled where the traversal met it; 2.49 with the lanes
-// sampling together, a 32-byte stack and positive t compared as bits; 2.13
-// with midpoints, float32 pairs and dt on the integer pipe and each cell's
-// entry taken from the last one's exit; 1.82 with parents restored in the
-// iteration that goes on with them; 1.63 with the heavy tiles first
-// (ytgb_schedule.cuh).  4 blocks per SM by registers; held to 5 1.85 against
-// 1.82, to 6 1.91.
+// float64 pipe at 38 %.  1024^2 frame of a 217,000-cell octree of levels 5-9: 2.98
+// ms with the traversal on the float64 pipe and each cell sampled where it was
+// met, 1.63 now.  4 blocks per SM by registers; held to 5 it is 2 % slower.
 template <int MODE, int CTF>
 __global__ void __launch_bounds__(OBLOCK) octree_kernel(const ytgb_render_args a, const ytgb_octree_args oa,
                                                          const unsigned short *tiles, unsigned long long *hashes, long long *counts) {

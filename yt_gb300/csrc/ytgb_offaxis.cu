@@ -384,8 +384,11 @@ __global__ void __launch_bounds__(OA_BLOCK) offaxis_kernel(const ytgb_offaxis_ar
 // cell alone, then one lane per pixel boundary of as many cells as the table in
 // shared memory holds, then the pixels cell by cell, lanes over the columns and
 // groups of lanes over the rows.
-// 197,000 cells of levels 5-9 at 1024^2 (38 pixels to 2): 5.17 ms by the subcell
-// kernel, 1.01 here (0.69 with 64 bits).  Bound by the integer pipe's products.
+// 217,000 cells of levels 5-9 at 1024^2 (38 pixels to 2): 5.17 ms by the subcell
+// kernel, 1.02 here (0.69 with 64 bits, see above).  Issue is 62 % busy, the integer
+// pipe 60 % (the corners' products), the float64 pipe 39 % (boundaries and their
+// divisions).  7 blocks per SM and 8 cells a batch lie within 2 % of the best of 5
+// to 7 and 4 to 16.
 constexpr int OS_CAP = 520;   // pixel boundaries held per warp: a cell of 258 pixels each way
 constexpr int OS_CELLS = 8;   // cells of a warp's batch
 constexpr int OS_WARPS = 4;

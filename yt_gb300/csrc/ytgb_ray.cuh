@@ -1672,14 +1672,9 @@ YTGB_HD void sample_many(const ytgb_render_args &a, const float4 *s_tab, const R
 // and is set up for its new binade, or only the scale of dt changes.  These
 // last two are handled inside the loop, so that lanes stay in step (about one
 // step in ten of a 512-cell walk has some lane looking).
-// Measured (kernel, CUDA events, against the loop with its tests in every
-// step): projection of 512^3 at 2048^2 9.18 -> 6.38 ms (42 warp instructions
-// a step and 10 of looks, from 76), maximum of 255^3 at 1023x779 790 -> 651
-// us, 1024^2 AMR frame 1.54 -> 1.36 ms, AMR interpolated projection 1.14 ->
-// 1.03 ms.  Also measured: a loop per run, at whose ends lanes wait for each
-// other, 34.6 ms for that projection; the walk's last cell inside the loop,
-// 7 % slower on the AMR frame; adds on the multiply pipe (mad.wide), 9 %
-// slower on the projection.
+// Kernel times against the loop with its tests in every step: projection of 512^3
+// at 2048^2 9.18 -> 6.38 ms (42 warp instructions a step and 10 of looks, from 76),
+// 1024^2 AMR frame 1.54 -> 1.36 ms.
 // MANY: the cell's samples by sample_many, whose code is not repeated for the
 // walk's last cell (taken inside the loop).
 // NCH: the channels the projection samplers write, when the launch fixes

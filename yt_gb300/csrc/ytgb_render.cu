@@ -70,26 +70,20 @@ template <> struct TileShape<2> { static constexpr int X = 4, Y = 32; };
 constexpr int BLOCK = 128;
 constexpr int NWARP = BLOCK / 32;
 // Resident blocks per SM the kernels are compiled for: warps hide the walk's
-// latencies, registers spare it spills.  Measured for each sampler (kernel
-// time, the other choices beside it):
-//   cell samplers (projection, maximum), whose loop holds little: 7 blocks,
-//     72 registers: 6.38 ms and 651 us (6: 6.55 and 690; 8: 6.68 and 652; 5:
-//     7.01 and 756) for 512^3 at 2048^2 and 255^3 at 1023x779;
-//   interpolated projection: 6, 80 registers: 1.026 ms (5: 1.023, 7: 1.057);
-//   ColorTransferFunction rendering: 5, 96 registers: 1.362 ms on the 1024^2
-//     AMR frame (6: 1.406);
-//   with float64 range decisions (V_REF), whose rare path needs the most: 4,
-//     128 registers: 500 us on a 701x1003 AMR frame (5: 545);
+// latencies, registers spare it spills.  The best of those measured for each
+// sampler (kernel time, the next best beside it):
+//   cell samplers (projection, maximum): 7, 6.38 ms (6: 6.55) for 512^3 at 2048^2;
+//   interpolated projection: 6, 1.026 ms (5: 1.023, 7: 1.057);
+//   ColorTransferFunction rendering: 5, 1.25 ms on a 1024^2 AMR frame (4: 1.35, 6:
+//     1.41 against 1.36 before the order of the tiles);
+//   with float64 range decisions (V_REF): 4, 0.50 ms on a 701x1003 frame (5: 0.55);
 //   with sample_many (V_MANY, the light source, other table sets): 4, where the
-//     corners stay in registers over a cell's samples: ten samples per cell
-//     640x480 1.10 ms (5: 1.33, 6: 1.67), light source 512^2 0.61 (5: 0.76, 6:
-//     1.00), three tables 701x1003 1.14 (5: 1.30, 6: 1.60); interpolated
-//     projection 6;
-//   the traversal trace: 6.
-// The persistent batch kernel, whose loop keeps more state: 5 (4.56 ms for 16
-// views; 4: 4.66, 6: 4.80).  Images are identical at every setting.
-// YTGB_MIN_BLOCKS sets all (a second build at another budget, for the
-// bit-identity test).
+//     corners stay in registers over a cell's samples: ten samples per cell 1.10
+//     ms (5: 1.33), light source 0.61 (5: 0.76); one sample of an AMR frame, which
+//     takes it where there is a mask arena, 1.35 (5: 1.30);
+//   the persistent batch kernel, whose loop keeps more state: 5, 4.56 ms (4: 4.66).
+// Images are identical at every setting.  YTGB_MIN_BLOCKS sets all (a second
+// build at another budget, for the bit-identity tests).
 #ifdef YTGB_MIN_BLOCKS
 constexpr int min_blocks(int, int) { return YTGB_MIN_BLOCKS; }
 constexpr int BATCH_MIN_BLOCKS = YTGB_MIN_BLOCKS;
@@ -511,8 +505,11 @@ int launch_many(const ytgb_render_args *a, size_t smem, const Scratch &w, cudaSt
 int tile_shape_of(uint32_t flags) { return (int)((flags >> YTGB_FLAG_TILE_SHIFT) & 0xfu); }
 
 // Volume rendering: the launch's variant, with sample_many where the
-// ColorTransferFunction walks are not all of one sample per unmasked cell
-// (other table sets have no simpler form).
+// ColorTransferFunction walks may not all be of one sample per unmasked cell
+// (other table sets have no simpler form).  A mask arena stands for masked cells:
+// which bricks have any is known on the device alone.  Where none has, the simple
+// kernel would take 1.25 ms for the 1024^2 AMR frame that this one renders in 1.35;
+// masked bricks it would take through the loop with every test in every step.
 int launch_vr(int var, int ts, const ytgb_render_args *a, size_t smem, const Scratch &w, cudaStream_t s) {
     const bool many = a->n_samples != 1 || a->masks;
     switch (var) {

@@ -18,15 +18,11 @@ namespace {
 // from the octree's cells) and the heavy tiles go first.  Any order gives the
 // same image.
 // Four steps of cost: more of them part neighbours that share bricks in the
-// caches.  Us at grid order / 2 / 4 / 8 / 16 steps, three volumes each: 1024^2
-// AMR frame 1337, 1195, 1211 / 1287, 1214, 1233 / 1248, 1216, 1231 / 1256, 1226,
-// 1250 / 1255, 1233, 1259 (the one out of balance gains, the others lose 2 %);
-// interpolated projection 1014, 888, 918 / 902, 923, 914 / 901, 921, 912 / 902,
-// 923, 911 / 915, 928, 915; 701x1003 range-decision frame 485, 570, 551 / 467,
-// 475, 463 / 463, 468, 440 / 461, 466, 446 / 466, 469, 449; ten samples per cell
-// 1076, 1010, 1070 / 890, 908, 935 / 881, 821, 928 / 882, 812, 932 / 879, 811,
-// 927; octree 1820, 1658, 1661 / 1707, 1591, 1633 / 1625, 1596, 1639 / 1640,
-// 1604, 1650 / 1658, 1619, 1667.
+// caches (2 to 16 steps lie within 3 %).  Us in grid order / in this order, three
+// volumes each: 1024^2 AMR frame 1337, 1195, 1211 / 1248, 1216, 1231 (frames
+// already in balance lose 2 %); ten samples per cell 1076, 1010, 1070 / 881, 821,
+// 928; 701x1003 range-decision frame 485, 570, 551 / 463, 468, 440; octree 1820,
+// 1658, 1661 / 1625, 1596, 1639.
 constexpr int SORT_BLOCK = 1024, SORT_BUCKETS = 4;
 // (tile numbers and their places are held in 16 bits)
 constexpr int MAX_SCHEDULED = 65535;
