@@ -35,3 +35,19 @@ def test_few_cells(cuda, n, monkeypatch):
         for g, r in zip(image, ref):
             assert bool(((g - r).abs() <= 1e-12 * r + 1e-24 * float(r.max())).all())
     assert n < 7 or float(ref[0].sum()) > 0  # (few cells may all lie beyond the image)
+
+
+@pytest.mark.parametrize("size", [(1, 1), (2, 3), (31, 31), (32, 33), (63, 200), (257, 257), (513, 700)])
+@pytest.mark.parametrize("width,n", [((2e-4, 5e-3), 1000), ((5e-3, 0.12), 333), ((0.25, 0.6), 5), ((1e-3, 0.3), 31)])
+def test_sums_of_few_cells(cuda, size, width, n):
+    """Cells from far below a pixel to wider than a warp's table of pixel
+    boundaries (518), on and across the image's edges, by the summed stamps,
+    which project() does not take for so few."""
+    nx, ny = size
+    rng = np.random.default_rng(nx + n)
+    dx = np.exp(rng.uniform(np.log(width[0]), np.log(width[1]), n))
+    x = rng.uniform(-0.7, 0.7, (n, 3))
+    rot = orientation(rng.standard_normal(3), rng.standard_normal(3))[0]
+    s = CellSplat(x, dx, rng.uniform(0.5, 2.0, n), rng.uniform(0.5, 2.0, n), device=cuda)
+    for g, r in zip(sums_image(s, rot, nx, ny), subcell_image(s, rot, nx, ny)):
+        assert bool(((g - r).abs() <= 1e-12 * r + 1e-24 * float(r.max())).all())
