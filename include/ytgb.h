@@ -431,8 +431,9 @@ void ytgb_octree_destroy(void *tree);
 int ytgb_render_octree(const ytgb_render_args *args, const ytgb_octree_args *o, void *stream);
 
 /* The same with scratch memory for the order of the blocks' tiles, as
- * ytgb_render_scheduled (ytgb_octree_scratch: 0 also for per-pixel rays). */
-int ytgb_octree_scratch(const ytgb_view *view, int32_t n_cells, int64_t *bytes);
+ * ytgb_render_scheduled (ytgb_octree_scratch: 0 also for per-pixel rays, few
+ * cells and a camera inside the domain). */
+int ytgb_octree_scratch(const ytgb_view *view, const ytgb_octree_args *o, int64_t *bytes);
 int ytgb_render_octree_scheduled(const ytgb_render_args *args, const ytgb_octree_args *o, void *scratch,
                                  int64_t bytes, void *stream);
 /* Traversal trace of the octree path: per pixel an FNV-1a hash over (cell

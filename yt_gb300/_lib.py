@@ -204,7 +204,7 @@ SIGNATURES = {
     "ytgb_octree_nodes": (C.c_int, [C.c_void_p, C.c_void_p]),
     "ytgb_octree_destroy": (None, [C.c_void_p]),
     "ytgb_render_octree": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p]),
-    "ytgb_octree_scratch": (C.c_int, [C.POINTER(View), C.c_int32, C.POINTER(C.c_int64)]),
+    "ytgb_octree_scratch": (C.c_int, [C.POINTER(View), C.c_void_p, C.POINTER(C.c_int64)]),
     "ytgb_render_octree_scheduled": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p]),
     "ytgb_offaxis_cells": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p]),
     "ytgb_offaxis_sums_bytes": (C.c_int, [C.c_int32] * 3 + [C.POINTER(C.c_int64)]),

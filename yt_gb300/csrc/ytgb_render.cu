@@ -429,14 +429,14 @@ tile_cost_kernel(const int4 *rects, const int32_t *order, const ytgb_brick *bric
 
 // The order of a launch's tiles in scratch memory, formed on its stream, or
 // null for grid order: without scratch memory for it, with one brick (its
-// tiles differ little), where all blocks are resident at once, and past
-// MAX_SCHEDULED tiles (the last blocks' time weighs little then).
+// tiles differ little), with no more blocks than two resident waves (ORDER_WAVES),
+// and past MAX_SCHEDULED tiles (the last blocks' time weighs little then).
 int schedule_tiles(const ytgb_render_args &a, int tx, int ty, int blocks_per_sm, const Scratch &w, cudaStream_t s,
                    const unsigned short **tiles) {
     *tiles = nullptr;
     const long long n = (long long)((a.view.nx + tx - 1) / tx) * ((a.view.ny + ty - 1) / ty);
     if (!w.mem || w.bytes < scratch_bytes(n) || a.n_order < 2 || n > MAX_SCHEDULED ||
-        n <= (long long)blocks_per_sm * sm_count())
+        n <= ORDER_WAVES * (long long)blocks_per_sm * sm_count())
         return YTGB_OK;
     unsigned *cost = (unsigned *)w.mem;
     cudaMemsetAsync(cost, 0, (size_t)n * sizeof(unsigned), s);
@@ -610,7 +610,7 @@ extern "C" int ytgb_render_scratch(const ytgb_view *view, int32_t n_order, int64
         const long long k = ((long long)view->nx + tx - 1) / tx * (((long long)view->ny + ty - 1) / ty);
         if (k <= MAX_SCHEDULED && k > n) n = k;
     }
-    *bytes = n_order < 2 || n <= 4 * sm_count() ? 0 : (int64_t)scratch_bytes(n);
+    *bytes = n_order < 2 || n <= ORDER_WAVES * 4 * sm_count() ? 0 : (int64_t)scratch_bytes(n);
     return YTGB_OK;
 }
 

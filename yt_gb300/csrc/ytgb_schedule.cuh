@@ -18,14 +18,19 @@ namespace {
 // from the octree's cells) and the heavy tiles go first.  Any order gives the
 // same image.
 // Four steps of cost: more of them part neighbours that share bricks in the
-// caches (2 to 16 steps lie within 3 %).  Us in grid order / in this order, three
-// volumes each: 1024^2 AMR frame 1337, 1195, 1211 / 1248, 1216, 1231 (frames
-// already in balance lose 2 %); ten samples per cell 1076, 1010, 1070 / 881, 821,
-// 928; 701x1003 range-decision frame 485, 570, 551 / 463, 468, 440; octree 1820,
-// 1658, 1661 / 1625, 1596, 1639.
+// caches (2 to 16 steps lie within 3 %).
 constexpr int SORT_BLOCK = 1024, SORT_BUCKETS = 4;
 // (tile numbers and their places are held in 16 bits)
 constexpr int MAX_SCHEDULED = 65535;
+// Forming the order takes some 30 us, so it is left out where that was not won
+// back: with no more tiles than two waves of resident blocks (800 tiles: 3 to 20 %
+// lost), with fewer cells of an octree (10,000: 0 to 13 % lost, with one scene 8 %
+// won) and from a camera inside it (5 to 14 % lost).  Where it is formed, time in
+// grid order / in this order over 90 octree and 132 AMR frames from 320^2 to 1600^2:
+// 1.05 on average, 0.92 (an almost uniform octree, 0.8 ms) to 1.43 (a camera from
+// which most of the image is empty).
+constexpr int ORDER_WAVES = 2;
+constexpr int ORDER_CELLS = 1 << 16;
 __device__ __forceinline__ int cost_bucket(unsigned c, float scale) {
     const int b = (int)((float)c * scale);
     return SORT_BUCKETS - 1 - (b < SORT_BUCKETS - 1 ? b : SORT_BUCKETS - 1);

@@ -71,6 +71,11 @@ class Octree:
         return self._nodes
 
 
+# ytgb_octree_scratch asks for none below this many cells (a tiny frame is spared
+# the call: 2 us of 55)
+ORDER_CELLS = 1 << 16
+
+
 class OctreeVolume:
     """An octree and its cells resident on the device.  ``cells`` is yt's
     (n, 14) float64 layout: 8 vertex values ((i,j,k) C order), left edge,
@@ -125,7 +130,7 @@ def render_octree(vol: OctreeVolume, view: _lib.View, kind: int, image: torch.Te
     """One ``ytgb_render_octree`` launch into ``image`` ((nx, ny, 4) float64
     device tensor, updated in place -- or a host array, on a device that
     reads and writes pageable host memory)."""
-    from .volume import _f64_contiguous, _ptr, device_reads_host, normalised_light
+    from .volume import _f64_contiguous, _ptr, device_reads_host, normalised_light, scratch_memory
 
     if isinstance(image, np.ndarray) and not device_reads_host(vol.device):
         raise ValueError("a host image needs a device that reads pageable host memory")
@@ -154,11 +159,10 @@ def render_octree(vol: OctreeVolume, view: _lib.View, kind: int, image: torch.Te
     s = stream or torch.cuda.current_stream(vol.device)
     L = _lib.lib()
     need = C.c_int64()
-    _lib.check(L.ytgb_octree_scratch(C.byref(view), vol.n_cells, C.byref(need)), "ytgb_octree_scratch")
-    mem = None
-    if need.value:
-        with torch.cuda.stream(s):  # (its memory goes back to this stream's later work alone)
-            mem = torch.empty(need.value, dtype=torch.uint8, device=vol.device)
+    # (an image in host memory keeps grid order: its writes cross the link to the CPU)
+    if vol.n_cells >= ORDER_CELLS and not isinstance(image, np.ndarray):
+        _lib.check(L.ytgb_octree_scratch(C.byref(view), C.byref(o), C.byref(need)), "ytgb_octree_scratch")
+    mem = scratch_memory(need.value, s, vol.device)
     _lib.check(L.ytgb_render_octree_scheduled(C.byref(a), C.byref(o), _ptr(mem), need.value,
                                               C.c_void_p(s.cuda_stream)), "ytgb_render_octree")
     return a, o

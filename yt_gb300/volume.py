@@ -487,6 +487,22 @@ def _view_key(view: _lib.View) -> bytes:
     return bytes(view)[: _lib.View.px_pos.offset]
 
 
+# The order of the tiles is formed from this many bricks on: frames of 135 and 165
+# bricks lost 2 to 20 % to it (30 us) but for one in ten, which won up to 17.
+ORDER_BRICKS = 256
+
+
+def scratch_memory(n: int, stream, device):
+    """n bytes of device memory (None for 0) that go back to ``stream``'s later
+    work alone."""
+    if n == 0:
+        return None
+    if stream == torch.cuda.current_stream(device):  # (entering a stream takes the host 10 us)
+        return torch.empty(n, dtype=torch.uint8, device=device)
+    with torch.cuda.stream(stream):
+        return torch.empty(n, dtype=torch.uint8, device=device)
+
+
 class RenderTables:
     """The table one render reads -- each order entry's pixel rectangle (4
     int32), then the order -- on the device, with the host copies of the
@@ -538,12 +554,9 @@ def render(bricks: BrickSet, view: _lib.View, order: np.ndarray, kind: int, imag
     L = _lib.lib()
     need = C.c_int64()
     # (an image in host memory keeps grid order: its writes cross the link to the CPU)
-    if not isinstance(image, np.ndarray):
+    if order.size >= ORDER_BRICKS and not isinstance(image, np.ndarray):
         _lib.check(L.ytgb_render_scratch(C.byref(view), order.size, C.byref(need)), "ytgb_render_scratch")
-    scratch = None
-    if need.value and (tables is not None or rects is not None):
-        with torch.cuda.stream(stream):  # (its memory goes back to this stream's later work alone)
-            scratch = torch.empty(need.value, dtype=torch.uint8, device=dev)
+    scratch = scratch_memory(need.value if tables is not None or rects is not None else 0, stream, dev)
     if tables is None and rects is None:
         tab_d = bricks.device_table(view, order, stream, need.value)
     elif tables is None:
