@@ -1,7 +1,7 @@
 """The same images at another register budget, for the single-view kernels that
 the library compiles for 4 resident blocks per SM (128 registers a thread):
 several samples per cell, masked bricks, the light source, other table sets,
-and float64 range decisions.
+and float64 range decisions, these also in a batch.
 
 tests/test_gpu_codegen.py compares the library with a build at 4 blocks, which
 for these kernels is the library's own budget; here the second build is at 5 (96
@@ -20,6 +20,7 @@ from test_gpu_codegen import CSRC, ROOT
 from test_kernel_host import near_bound_case
 from yt_gb300 import _lib, testing, workloads
 from yt_gb300.amr_kdtree import AMRKDTree
+from yt_gb300.batch import Batch, Job
 from yt_gb300.camera import Camera
 from yt_gb300.render import Renderer
 from yt_gb300.volume import BrickSet
@@ -90,3 +91,31 @@ def test_single_view_kernels_at_another_budget(cuda, other):
     for (r, cam, kind, ns), a, b in zip(work, want, got):
         assert same_bits(a, b), (kind, ns)
     assert all(float(torch.nan_to_num(a).abs().max()) > 0 for a in want)
+
+
+def test_batch_range_decisions_at_another_budget(cuda, other):
+    near, near_tf = near_bound_case()
+    light = ((-0.3, 0.8, 0.2), (0.9, 0.5, 0.2, 1.0))
+    r = {k: Renderer(BrickSet(near, device=cuda, with_lo=True), near_tf[k], device=cuda) for k in ("ctf", "general")}
+    V, S = _lib.VOLUME_RENDER, _lib.LIGHT_SOURCE
+    jobs = [Job(r[k], cam, kind, n_samples=ns, light=light if kind == S else None)
+            for k, kind, ns in (("ctf", V, 1), ("ctf", V, 3), ("general", V, 1), ("general", V, 2), ("ctf", S, 2))
+            for cam in cams(3, seed=4)]
+    b = Batch(jobs, device=cuda)
+    b.launch()
+    torch.cuda.synchronize()
+    b.check()
+    want = [im.clone() for im in b.images]
+    for im in b.images:
+        im.zero_()
+    stream = torch.cuda.current_stream(cuda)
+    for q, g in enumerate(b.groups):
+        st = other.ytgb_batch_render(g.dev.data_ptr(), g.n, g.kind, g.variant, b.tile_shape, g.total_tiles, g.smem,
+                                     b.queue.data_ptr() + 4 * q, 0, C.c_void_p(stream.cuda_stream))
+        assert st == _lib.OK, other.ytgb_last_error()
+    torch.cuda.synchronize()
+    b.check()
+    for j, im in zip(jobs, want):
+        assert same_bits(j.image, im), (j.kind, j.n_samples)
+        one = j.renderer.render(j.camera, kind=j.kind, n_samples=j.n_samples, light=j.light)
+        assert same_bits(one, im), (j.kind, j.n_samples)

@@ -81,12 +81,13 @@ constexpr int NWARP = BLOCK / 32;
 //     corners stay in registers over a cell's samples: ten samples per cell 1.10
 //     ms (5: 1.33), light source 0.61 (5: 0.76); one sample of an AMR frame, which
 //     takes it where there is a mask arena, 1.35 (5: 1.30);
-//   the persistent batch kernel, whose loop keeps more state: 5, 4.56 ms (4: 4.66).
+//   the persistent batch kernel, whose loop keeps more state: 5, 4.56 ms (4: 4.66);
+//     with V_REF 4: two samples 2.47 ms (5: 2.75), light source 4.62 (5: 6.24).
 // Images are identical at every setting.  YTGB_MIN_BLOCKS sets all (a second
 // build at another budget, for the bit-identity tests).
 #ifdef YTGB_MIN_BLOCKS
 constexpr int min_blocks(int, int) { return YTGB_MIN_BLOCKS; }
-constexpr int BATCH_MIN_BLOCKS = YTGB_MIN_BLOCKS;
+constexpr int batch_min_blocks(int) { return YTGB_MIN_BLOCKS; }
 #else
 constexpr int min_blocks(int mode, int var) {
     return mode == MODE_PROJ || mode == MODE_MIP ? 7
@@ -95,7 +96,7 @@ constexpr int min_blocks(int mode, int var) {
            : (var & V_CTF)                       ? 5
                                                  : 6;
 }
-constexpr int BATCH_MIN_BLOCKS = 5;
+constexpr int batch_min_blocks(int var) { return (var & V_REF) ? 4 : 5; }
 #endif
 
 // Selected bricks a warp holds before walking them (flushed in order when
@@ -253,7 +254,7 @@ render_kernel(const ytgb_render_args a, const unsigned short *tiles, unsigned lo
 // loop iteration takes a new item: a warp runs at most as many iterations as
 // there are items (no spin, and no barrier after the staging).
 template <int MODE, int VAR, int TS, bool STAGED>
-__global__ void __launch_bounds__(BLOCK, BATCH_MIN_BLOCKS) batch_kernel(const ytgb_batch_entry *entries, int n_entries,
+__global__ void __launch_bounds__(BLOCK, batch_min_blocks(VAR)) batch_kernel(const ytgb_batch_entry *entries, int n_entries,
                                                       int total_tiles, int *queue) {
     extern __shared__ float4 s_tab[];
     __shared__ TileSmem sm;
